@@ -1107,50 +1107,53 @@ rocblas_status trtri_impl(rocblas_handle h, rocblas_fill uplo, rocblas_diagonal 
         h->pointer_mode = mode;
         return st;
     }
-    const size_t ws_bytes = trtri_workspace_bytes<T>(n, std::max(batch, 0));
-    if(h->size_query)
+    else
     {
-        if(!n || !ws_bytes)
-            return rocblas_status_size_unchanged;
-        return h->set_optimal_size(ws_bytes);
-    }
-    rocblas_status st = trtri_arg_check(uplo, diag, n, Aptr, lda, Xptr, ldinv, batch);
-    if(st != rocblas_status_continue)
-        return st;
-    if((st = device_ready(h)) != rocblas_status_success)
-        return st;
-    void* ws = nullptr;
-    if(ws_bytes && !(ws = h->borrow(ws_bytes)))
-        return rocblas_status_memory_error;
+        const size_t ws_bytes = trtri_workspace_bytes<T>(n, std::max(batch, 0));
+        if(h->size_query)
+        {
+            if(!n || !ws_bytes)
+                return rocblas_status_size_unchanged;
+            return h->set_optimal_size(ws_bytes);
+        }
+        rocblas_status st = trtri_arg_check(uplo, diag, n, Aptr, lda, Xptr, ldinv, batch);
+        if(st != rocblas_status_continue)
+            return st;
+        if((st = device_ready(h)) != rocblas_status_success)
+            return st;
+        void* ws = nullptr;
+        if(ws_bytes && !(ws = h->borrow(ws_bytes)))
+            return rocblas_status_memory_error;
 
-    TrtriParams<T> t{};
-    t.k = n;
-    t.nb = kInvNB;
-    t.A = A;
-    t.lda = lda;
-    t.inv = X;
-    t.ldinv = ldinv;
-    t.inv_block_stride = (int64_t)kInvNB * ldinv + kInvNB;
-    t.upper = uplo == rocblas_fill_upper;
-    t.unit = diag == rocblas_diagonal_unit;
-    launch_trtri<T>(t, (int)ceil_div(n, kInvNB), batch, h->stream);
-    if(n > kInvNB)
-    {
-        TrtriRec<T> r;
-        r.n = n;
-        r.upper = t.upper;
-        r.A = A;
-        r.X = X;
-        r.lda = lda;
-        r.ldx = ldinv;
-        const int64_t half = ceil_div(ceil_div(n, kInvNB), 2) * kInvNB;
-        r.Tmp = strided<T>(reinterpret_cast<T*>(ws), half * half);
-        r.ldt = 0;
-        r.batch = batch;
-        r.s = h->stream;
-        r.run(0, (int)ceil_div(n, kInvNB));
+        TrtriParams<T> t{};
+        t.k = n;
+        t.nb = kInvNB;
+        t.A = A;
+        t.lda = lda;
+        t.inv = X;
+        t.ldinv = ldinv;
+        t.inv_block_stride = (int64_t)kInvNB * ldinv + kInvNB;
+        t.upper = uplo == rocblas_fill_upper;
+        t.unit = diag == rocblas_diagonal_unit;
+        launch_trtri<T>(t, (int)ceil_div(n, kInvNB), batch, h->stream);
+        if(n > kInvNB)
+        {
+            TrtriRec<T> r;
+            r.n = n;
+            r.upper = t.upper;
+            r.A = A;
+            r.X = X;
+            r.lda = lda;
+            r.ldx = ldinv;
+            const int64_t half = ceil_div(ceil_div(n, kInvNB), 2) * kInvNB;
+            r.Tmp = strided<T>(reinterpret_cast<T*>(ws), half * half);
+            r.ldt = 0;
+            r.batch = batch;
+            r.s = h->stream;
+            r.run(0, (int)ceil_div(n, kInvNB));
+        }
+        return launch_status();
     }
-    return launch_status();
 }
 
 __global__ void vb_copy_invalid_kernel(const int* invalid, rocblas_int* out)

@@ -119,6 +119,7 @@ static void launch_gemm(const GemmParams<T>& p0, int batch, cudaStream_t s, int 
 template <typename T>
 static void launch_trtri(const TrtriParams<T>& p0, int nblocks, int batch, cudaStream_t s)
 {
+    static_assert(!is_cplx<T>::value, "complex solves build no inverse blocks");
     const size_t smem = trtri_smem_bytes<T>();
     ensure_smem_attr<T>((const void*)trtri_block_kernel<T>, smem);
     for(int b0 = 0; b0 < batch; b0 += kMaxGridYZ)

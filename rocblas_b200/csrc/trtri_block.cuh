@@ -3,14 +3,20 @@
 // Replaces the reference's invA construction for TRSM (rocblas_trtri_trsm_template,
 // library/src/blas3/trtri_trsm.hpp:110-381: 16x16 trtri kernels, three rounds of
 // strided-batched GEMM merges 32->64->128, a separate fill kernel for the unused
-// triangle and a remainder trtri) with a single fused kernel: the block (at most 128 x 128)
-// is staged in shared memory as 4 x 4 tiles of 32 x 32 (lower orientation; an upper block U
-// is handled as the lower block J U J, J the exchange matrix), the four diagonal tiles are
-// inverted by four warps (lane = column, substitution in registers, A entries broadcast
-// from shared memory), and the off-diagonal tiles follow by diagonal distance d = 1, 2, 3:
-//     X(i,j) = -X(i,i) * sum_{t=j}^{i-1} L(i,t) X(t,j).
-// The result, with zeros in the opposite triangle (what rocblas_trtri_fill does,
-// rocblas_trtri.hpp:393-426), is written to invA.
+// triangle and a remainder trtri) with a single fused kernel: the block (at most 128 x 128,
+// padded with the identity) is staged in shared memory in lower orientation (an upper block U
+// is handled as the lower block J U J, J the exchange matrix), its eight 16 x 16 diagonal
+// tiles are inverted by one warp each (lane = column, substitution in registers), and the
+// inverses of 32, 64 and 128 rows follow in place from
+//     [[L11, 0], [L21, L22]]^-1 = [[X11, 0], [-X22 L21 X11, X22]],
+// two DMMA products per doubling that skip the zero halves of X11 and X22.  The result, with
+// zeros in the opposite triangle (what rocblas_trtri_fill does, rocblas_trtri.hpp:393-426), is
+// written to invA.  FP32 blocks are inverted in FP64 and rounded once.
+//
+// The kernel is a chain of short steps (a solve waits for it before its first block), so it is
+// bound by latency: copies that are all in flight at once, seven CTA barriers, and no index
+// arithmetic beyond constants: about 9 us for up to 148 blocks of 128 where the version on 32 x 32
+// tiles with computed tile indexes took 42 us (a third of a 512 x 256 solve).
 //
 // Diagonal semantics follow rocblas_custom_trtri_device (rocblas_trtri.hpp:128-141):
 // diag == unit reads no diagonal and uses 1; a zero non-unit diagonal entry is treated as 1.
@@ -18,6 +24,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "mbarrier.cuh"
 #include "mma_f64.cuh"
 
 namespace rb200
@@ -42,63 +49,49 @@ struct TrtriParams
 };
 
 constexpr int kTrtriNB      = 128;
-constexpr int kTrtriSB      = 32;  // tile order
-constexpr int kTrtriNT      = 4;   // tiles per side
-constexpr int kTrtriNTiles  = kTrtriNT * (kTrtriNT + 1) / 2; // 10 lower tiles
-constexpr int kTrtriThreads = 256;
-
-// Tile row pitch in shared memory: 33 keeps the column reads of the FMA products
-// conflict-free; FP64 runs the products on DMMA, whose fragment reads (lanes (g, t) reading
-// (g, t) of the left tile and (t, g) of the right one) need a pitch of 4 mod 16.
-template <typename T>
-__host__ __device__ constexpr int trtri_pitch()
-{
-    return std::is_same<T, double>::value ? 36 : 33;
-}
-template <typename T>
-__host__ __device__ constexpr int trtri_tile()
-{
-    return kTrtriSB * trtri_pitch<T>();
-}
+constexpr int kTrtriThreads = 256; // 8 warps
+// Column pitch in shared memory (column-major): the fragment reads, lanes (g, t) at element (g, t)
+// or (t, g), are free of bank conflicts with a pitch of 4 mod 16 doubles.
+constexpr int kTrtriLd  = kTrtriNB + 4;
+constexpr int kTrtriLdT = kTrtriNB / 2 + 4; // temporary of at most 64 x 64
 
 template <typename T>
 constexpr size_t trtri_smem_bytes()
 {
-    // L tiles, X tiles, 3 temporaries, reciprocal diagonal
-    return sizeof(T) * (size_t)(2 * kTrtriNTiles * trtri_tile<T>() + 3 * trtri_tile<T>() + kTrtriNB);
+    return sizeof(double) * (size_t)(kTrtriNB * kTrtriLd + kTrtriNB / 2 * kTrtriLdT);
 }
 
-// acc (the 16 x 8 block of warp (wr, wc) of a 32 x 32 tile product) += Lt Rt, FP64 DMMA.
-__device__ __forceinline__ void trtri_tile_mma(double (&acc)[4], const double* Lt, const double* Rt,
-                                               int wr, int wc, int g, int t)
+// NT neighbouring 16 x 8 tiles acc[n] += P(r0.., k) Q(k, c0 + 8n ..) over k in [k0, k1); P and Q
+// column-major with pitches ldp, ldq.
+template <int NT>
+__device__ __forceinline__ void trtri_mma(double (&acc)[NT][4], const double* P, int ldp, const double* Q, int ldq,
+                                          int k0, int k1, int g, int t)
 {
-    constexpr int P = 36;
-#pragma unroll
-    for(int ks = 0; ks < kTrtriSB; ks += 8)
+#pragma unroll 2
+    for(int k = k0; k < k1; k += 8)
     {
-        const double a[4] = {Lt[(wr + g) * P + ks + t], Lt[(wr + g + 8) * P + ks + t],
-                             Lt[(wr + g) * P + ks + t + 4], Lt[(wr + g + 8) * P + ks + t + 4]};
-        const double b[2] = {Rt[(ks + t) * P + wc + g], Rt[(ks + t + 4) * P + wc + g]};
-        dmma_16x8x8(acc, a, b);
+        const double* a0 = P + (k + t) * ldp + g;
+        const double* a1 = P + (k + t + 4) * ldp + g;
+        const double  a[4] = {a0[0], a0[8], a1[0], a1[8]};
+#pragma unroll
+        for(int n = 0; n < NT; ++n)
+        {
+            const double* q    = Q + (8 * n + g) * ldq + k + t;
+            const double  b[2] = {q[0], q[4]};
+            dmma_16x8x8(acc[n], a, b);
+        }
     }
-}
-
-__device__ __forceinline__ int trtri_tile_index(int bi, int bj)
-{
-    return bi * (bi + 1) / 2 + bj;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<T> p)
 {
-    constexpr int kTrtriPitch = trtri_pitch<T>(), kTrtriTile = trtri_tile<T>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* Ls    = reinterpret_cast<T*>(smem_raw);
-    T* Xs    = Ls + kTrtriNTiles * kTrtriTile;
-    T* Ts    = Xs + kTrtriNTiles * kTrtriTile;
-    T* rdiag = Ts + 3 * kTrtriTile;
+    double* X  = reinterpret_cast<double*>(smem_raw); // the block, then its inverse in place
+    double* Tm = X + kTrtriNB * kTrtriLd;
 
-    const int     tid   = threadIdx.x;
+    const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int     g = lane >> 2, t = lane & 3;
     const int     blk   = blockIdx.x;
     const int     batch = p.batch_base + blockIdx.y;
     const int     k     = p.vk ? p.vk[batch] : p.k;
@@ -110,187 +103,110 @@ __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<
 
     const T* A   = p.A.get(batch) + r0 + (int64_t)r0 * lda;
     T*       out = p.inv.get(batch) + (int64_t)blk * p.inv_block_stride;
+    // (i, j) of the lower orientation is A(i, j), or A(bs - 1 - i, bs - 1 - j) of an upper block
+    const T* const A0 = p.upper ? A + (int64_t)(bs - 1) * (lda + 1) : A;
+    const int      sg = p.upper ? -1 : 1;
 
-    // ---- stage the block in lower orientation, identity-padded to 128 ----------------
-    // The 10 lower 32 x 32 tiles, 40 elements per thread, row index fastest so that a lower
-    // block is read down its columns; loads are issued 8 at a time before their stores.
+    // ---- stage the lower triangle, identity-padded to 128 -----------------------------------
+    // Warp w takes the columns w, w + 8, ..; whole 32-row groups above the diagonal are left out.
+#pragma unroll
+    for(int c = 0; c < kTrtriNB / 8; ++c)
     {
-        constexpr int kPer = kTrtriNTiles * kTrtriSB * kTrtriSB / kTrtriThreads; // 40
-        constexpr int kBatch = 8;
-        static_assert(kPer % kBatch == 0, "staging batches");
-        auto coords = [&](int e, int& tl, int& i, int& j) {
-            tl = e >> 10; // tile in trtri_tile_index order
-            int bi = 0;
-            while(trtri_tile_index(bi + 1, 0) <= tl)
-                ++bi;
-            const int bj = tl - trtri_tile_index(bi, 0);
-            i = bi * kTrtriSB + (e & 31);
-            j = bj * kTrtriSB + ((e >> 5) & 31);
-        };
-#pragma unroll 1
-        for(int u0 = 0; u0 < kPer; u0 += kBatch)
+        const int j = c * 8 + warp;
+#pragma unroll
+        for(int u = c / 4; u < kTrtriNB / 32; ++u)
         {
-            T v[kBatch];
-#pragma unroll
-            for(int u = 0; u < kBatch; ++u)
-            {
-                int tl, i, j;
-                coords(tid + (u0 + u) * kTrtriThreads, tl, i, j);
-                v[u] = T(0);
-                if(j <= i && i < bs && j < bs && !(i == j && p.unit))
-                {
-                    const int r = p.upper ? bs - 1 - i : i;
-                    const int c = p.upper ? bs - 1 - j : j;
-                    v[u] = A[r + (int64_t)c * lda];
-                }
-            }
-#pragma unroll
-            for(int u = 0; u < kBatch; ++u)
-            {
-                int tl, i, j;
-                coords(tid + (u0 + u) * kTrtriThreads, tl, i, j);
-                T x = v[u];
-                if(i == j)
-                {
-                    // unit diagonal, identity padding, and a zero diagonal entry read as 1
-                    if(p.unit || i >= bs || x == T(0))
-                        x = T(1);
-                    rdiag[i] = T(1) / x;
-                }
-                Ls[tl * kTrtriTile + (i % kTrtriSB) * kTrtriPitch + (j % kTrtriSB)] = x;
-            }
+            const int  i    = u * 32 + lane;
+            const bool take = i < bs && j < bs && (j < i || (i == j && !p.unit));
+            const T*   src  = take ? A0 + sg * (i + (int64_t)j * lda) : A0;
+            double*    dst  = X + j * kTrtriLd + i;
+            if constexpr(std::is_same<T, double>::value)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
+                             "r"(take ? 8 : 0)
+                             : "memory");
+            else
+                *dst = take ? (double)*src : 0.0;
         }
     }
-    __syncthreads();
-
-    // ---- invert the four diagonal tiles: warp w < 4 takes tile w, lane = column -------
-    {
-        const int w = tid >> 5, lane = tid & 31;
-        if(w < kTrtriNT)
-        {
-            const T* L = Ls + trtri_tile_index(w, w) * kTrtriTile;
-            T        x[kTrtriSB];
-#pragma unroll
-            for(int i = 0; i < kTrtriSB; ++i)
-                x[i] = (i == lane) ? T(1) : T(0);
-#pragma unroll
-            for(int t = 0; t < kTrtriSB; ++t)
-            {
-                x[t] *= rdiag[w * kTrtriSB + t];
-#pragma unroll
-                for(int i = t + 1; i < kTrtriSB; ++i)
-                    x[i] -= L[i * kTrtriPitch + t] * x[t];
-            }
-            T* X = Xs + trtri_tile_index(w, w) * kTrtriTile;
-#pragma unroll
-            for(int i = 0; i < kTrtriSB; ++i)
-                X[i * kTrtriPitch + lane] = x[i];
-        }
-    }
-    __syncthreads();
-
-    // ---- off-diagonal tiles by distance d ------------------------------------------------
-    const int c  = tid & 31;   // tile column handled by this thread
-    const int rb = tid >> 5;   // rows rb, rb+8, rb+16, rb+24
     if constexpr(std::is_same<T, double>::value)
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+
+    // ---- 16 x 16 diagonal tiles: warp w inverts tile w, lane = column ----------------------------
     {
-        // FP64: both products on DMMA, warp w owns the 16 x 8 block at rows 16 (w % 2),
-        // columns 8 (w / 2) of each 32 x 32 tile
-        const int lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
-        const int wr = (w & 1) * 16, wc = (w >> 1) * 8;
-        for(int d = 1; d < kTrtriNT; ++d)
+        constexpr int S = 16;
+        double* const D = X + warp * S * (kTrtriLd + 1);
+        double        d = lane < S ? D[lane * (kTrtriLd + 1)] : 1.0;
+        // unit diagonal and padding (staged as 0), and a zero diagonal entry, read as 1
+        d = d == 0.0 ? 1.0 : d;
+        const double rd = 1.0 / d;
+        double       x[S];
+#pragma unroll
+        for(int i = 0; i < S; ++i)
+            x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+        for(int c = 0; c < S; ++c)
         {
-            const int npairs = kTrtriNT - d;
-            for(int pr = 0; pr < npairs; ++pr)
-            {
-                const int bj = pr, bi = pr + d;
-                double    acc[4] = {0.0, 0.0, 0.0, 0.0};
-                for(int bt = bj; bt < bi; ++bt)
-                    trtri_tile_mma(acc, Ls + trtri_tile_index(bi, bt) * kTrtriTile,
-                                   Xs + trtri_tile_index(bt, bj) * kTrtriTile, wr, wc, g, t);
+            x[c] *= __shfl_sync(0xffffffffu, rd, c);
 #pragma unroll
-                for(int e = 0; e < 4; ++e)
-                    Ts[pr * kTrtriTile + (wr + g + (e >> 1) * 8) * kTrtriPitch + wc + 2 * t + (e & 1)]
-                        = acc[e];
-            }
-            __syncthreads();
-            for(int pr = 0; pr < npairs; ++pr)
-            {
-                const int bj = pr, bi = pr + d;
-                double    acc[4] = {0.0, 0.0, 0.0, 0.0};
-                trtri_tile_mma(acc, Xs + trtri_tile_index(bi, bi) * kTrtriTile, Ts + pr * kTrtriTile,
-                               wr, wc, g, t);
-                T* Xo = Xs + trtri_tile_index(bi, bj) * kTrtriTile;
-#pragma unroll
-                for(int e = 0; e < 4; ++e)
-                    Xo[(wr + g + (e >> 1) * 8) * kTrtriPitch + wc + 2 * t + (e & 1)] = -acc[e];
-            }
-            __syncthreads();
+            for(int i = c + 1; i < S; ++i)
+                x[i] -= D[c * kTrtriLd + i] * x[c];
         }
+        __syncwarp();
+        if(lane < S)
+#pragma unroll
+            for(int i = 0; i < S; ++i)
+                D[lane * kTrtriLd + i] = x[i];
     }
-    else
-    for(int d = 1; d < kTrtriNT; ++d)
-    {
-        const int npairs = kTrtriNT - d;
-        // T_p = sum_{t=j}^{i-1} L(i,t) X(t,j),   (i, j) = (j + d, j), j = p
-        for(int pr = 0; pr < npairs; ++pr)
-        {
-            const int bj = pr, bi = pr + d;
-            T         acc[4] = {T(0), T(0), T(0), T(0)};
-            for(int bt = bj; bt < bi; ++bt)
+    __syncthreads();
+
+    // ---- 16 -> 32 -> 64 -> 128 ----------------------------------------------------------------
+    // Of a doubling from S, the warp takes NT tiles of 16 x 8 at row rb, column cb of pair pr.
+    auto doubling = [&](auto s_const, auto nt_const, int pr, int rb, int cb) {
+        constexpr int S = decltype(s_const)::value, NT = decltype(nt_const)::value;
+        double* const X11 = X + pr * 2 * S * (kTrtriLd + 1);
+        double* const L21 = X11 + S;
+        double* const X22 = X11 + S * (kTrtriLd + 1);
+        double* const Tp  = Tm + pr * S * kTrtriLdT; // its S columns of the temporary
+        double        acc[NT][4] = {};
+        // Tp = L21 X11: X11's column c is zero above row c
+        trtri_mma<NT>(acc, L21 + rb, kTrtriLd, X11 + cb * kTrtriLd, kTrtriLd, cb, S, g, t);
+#pragma unroll
+        for(int n = 0; n < NT; ++n)
+#pragma unroll
+            for(int e = 0; e < 4; ++e)
             {
-                const T* L = Ls + trtri_tile_index(bi, bt) * kTrtriTile;
-                const T* X = Xs + trtri_tile_index(bt, bj) * kTrtriTile;
-#pragma unroll 8
-                for(int kk = 0; kk < kTrtriSB; ++kk)
-                {
-                    const T xv = X[kk * kTrtriPitch + c];
-#pragma unroll
-                    for(int q = 0; q < 4; ++q)
-                        acc[q] += L[(rb + 8 * q) * kTrtriPitch + kk] * xv;
-                }
+                Tp[(cb + 8 * n + 2 * t + (e & 1)) * kTrtriLdT + rb + g + (e >> 1) * 8] = acc[n][e];
+                acc[n][e] = 0.0;
             }
-#pragma unroll
-            for(int q = 0; q < 4; ++q)
-                Ts[pr * kTrtriTile + (rb + 8 * q) * kTrtriPitch + c] = acc[q];
-        }
         __syncthreads();
-        // X(i,j) = -X(i,i) T_p
-        for(int pr = 0; pr < npairs; ++pr)
-        {
-            const int bj = pr, bi = pr + d;
-            const T*  Xd = Xs + trtri_tile_index(bi, bi) * kTrtriTile;
-            const T*  Tp = Ts + pr * kTrtriTile;
-            T         acc[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll 8
-            for(int kk = 0; kk < kTrtriSB; ++kk)
-            {
-                const T tv = Tp[kk * kTrtriPitch + c];
+        // X21 = -X22 Tp, over L21: X22's row r ends at column r
+        trtri_mma<NT>(acc, X22 + rb, kTrtriLd, Tp + cb * kTrtriLdT, kTrtriLdT, 0, rb + 16, g, t);
 #pragma unroll
-                for(int q = 0; q < 4; ++q)
-                    acc[q] += Xd[(rb + 8 * q) * kTrtriPitch + kk] * tv;
-            }
-            T* Xo = Xs + trtri_tile_index(bi, bj) * kTrtriTile;
+        for(int n = 0; n < NT; ++n)
 #pragma unroll
-            for(int q = 0; q < 4; ++q)
-                Xo[(rb + 8 * q) * kTrtriPitch + c] = -acc[q];
-        }
+            for(int e = 0; e < 4; ++e)
+                L21[(cb + 8 * n + 2 * t + (e & 1)) * kTrtriLd + rb + g + (e >> 1) * 8] = -acc[n][e];
         __syncthreads();
-    }
+    };
+    doubling(std::integral_constant<int, 16>{}, std::integral_constant<int, 1>{}, warp >> 1, 0, (warp & 1) * 8);
+    doubling(std::integral_constant<int, 32>{}, std::integral_constant<int, 2>{}, warp >> 2, (warp & 1) * 16,
+             (warp & 2) * 8);
+    // warps w and w + 4 share a scheduler: opposite row blocks give it even work in both products
+    doubling(std::integral_constant<int, 64>{}, std::integral_constant<int, 4>{}, 0,
+             (warp < 4 ? warp : 7 - warp) * 16, (warp >> 2) * 32);
 
     // ---- write inv(A_block) (bs x bs, ld = ldinv), zeros in the opposite triangle ----
-    for(int idx = tid; idx < bs * bs; idx += kTrtriThreads)
-    {
-        const int i = idx % bs, j = idx / bs;
-        // lower-orientation coordinates
-        const int li = p.upper ? bs - 1 - i : i;
-        const int lj = p.upper ? bs - 1 - j : j;
-        T         v  = T(0);
-        if(li >= lj)
-            v = Xs[trtri_tile_index(li / kTrtriSB, lj / kTrtriSB) * kTrtriTile
-                   + (li % kTrtriSB) * kTrtriPitch + (lj % kTrtriSB)];
-        out[i + (int64_t)j * p.ldinv] = v;
-    }
+    T* const out0 = p.upper ? out + (int64_t)(bs - 1) * (p.ldinv + 1) : out;
+#pragma unroll 4
+    for(int j = warp; j < bs; j += 8)
+#pragma unroll
+        for(int u = 0; u < kTrtriNB / 32; ++u)
+        {
+            const int i = u * 32 + lane;
+            if(i < bs)
+                out0[sg * (i + (int64_t)j * p.ldinv)] = i >= j ? (T)X[j * kTrtriLd + i] : T(0);
+        }
 }
 
 } // namespace rb200
