@@ -15,7 +15,7 @@
 //
 // The kernel is a chain of short steps (a solve waits for it before its first block), so it is
 // bound by latency: copies that are all in flight at once, seven CTA barriers, and no index
-// arithmetic beyond constants: about 9 us for up to 148 blocks of 128 where the version on 32 x 32
+// arithmetic beyond constants: 14 us for up to 148 FP64 blocks of 128 where the version on 32 x 32
 // tiles with computed tile indexes took 42 us (a third of a 512 x 256 solve).
 //
 // Diagonal semantics follow rocblas_custom_trtri_device (rocblas_trtri.hpp:128-141):
@@ -109,27 +109,45 @@ __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<
 
     // ---- stage the lower triangle, identity-padded to 128 -----------------------------------
     // Warp w takes the columns w, w + 8, ..; whole 32-row groups above the diagonal are left out.
-#pragma unroll
-    for(int c = 0; c < kTrtriNB / 8; ++c)
+    auto source = [&](int i, int j, bool& take) {
+        take = i < bs && j < bs && (j < i || (i == j && !p.unit));
+        return take ? A0 + sg * (i + (int64_t)j * lda) : A0;
+    };
+    if constexpr(std::is_same<T, double>::value)
     {
-        const int j = c * 8 + warp;
 #pragma unroll
-        for(int u = c / 4; u < kTrtriNB / 32; ++u)
-        {
-            const int  i    = u * 32 + lane;
-            const bool take = i < bs && j < bs && (j < i || (i == j && !p.unit));
-            const T*   src  = take ? A0 + sg * (i + (int64_t)j * lda) : A0;
-            double*    dst  = X + j * kTrtriLd + i;
-            if constexpr(std::is_same<T, double>::value)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
-                             "r"(take ? 8 : 0)
+        for(int c = 0; c < kTrtriNB / 8; ++c)
+#pragma unroll
+            for(int u = c / 4; u < kTrtriNB / 32; ++u)
+            {
+                const int i = u * 32 + lane, j = c * 8 + warp;
+                bool      take;
+                const T*  src = source(i, j, take);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(X + j * kTrtriLd + i)),
+                             "l"(src), "r"(take ? 8 : 0)
                              : "memory");
-            else
-                *dst = take ? (double)*src : 0.0;
+            }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    else
+    {
+        // converted on the way: a row group's loads are all issued before its stores
+#pragma unroll
+        for(int u = 0; u < kTrtriNB / 32; ++u)
+        {
+            T v[4 * (kTrtriNB / 32)];
+#pragma unroll
+            for(int c = 0; c < 4 * (u + 1); ++c)
+            {
+                bool     take;
+                const T* src = source(u * 32 + lane, c * 8 + warp, take);
+                v[c]         = take ? *src : T(0);
+            }
+#pragma unroll
+            for(int c = 0; c < 4 * (u + 1); ++c)
+                X[(c * 8 + warp) * kTrtriLd + u * 32 + lane] = (double)v[c];
         }
     }
-    if constexpr(std::is_same<T, double>::value)
-        asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
     // ---- 16 x 16 diagonal tiles: warp w inverts tile w, lane = column ----------------------------
