@@ -26,11 +26,11 @@ HEADERS = [HEADER, EXT_HEADER]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
-    "-O3", "-lineinfo", "-std=c++17",
+    "-O3", "-lineinfo", "-std=c++17", "--threads", "0",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
     "-shared",
 ]
-SOURCES = ["rocblas_api.cu"]
+SOURCES = ["rocblas_api.cu", "chain_kernels.cu", "tile_kernels.cu"]
 
 # ---- enums (include/rocblas.h; library/include/internal/rocblas-types.h:123-234) ---------
 operation_none, operation_transpose, operation_conjugate_transpose = 111, 112, 113

@@ -98,9 +98,9 @@ def tune(quick=False, out_dir=HERE):
     report["entries"]["chain_max_cols"] = {"chosen": _pick(res), "ms_sum_over_shapes": res,
                                            "shapes": shapes}
 
-    # ---- chain strip width (0: 32 up to 32 columns, else 64) --------------------------------
+    # ---- chain strip width (0: the library's cost model per call) -----------------------------
     res = {}
-    for c in [0, 32, 64]:
+    for c in [0, 8, 16, 32, 64]:
         set_tuning("chain_w", c)
         res[c] = plain_sum()
     set_tuning("chain_w", _pick(res))

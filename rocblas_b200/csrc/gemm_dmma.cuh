@@ -305,7 +305,7 @@ enum class DmmaTile
 constexpr int kDmmaTiles = 11;
 
 template <bool KCP, bool KCQ>
-static void launch_dmma_tile(DmmaTile t, const GemmParams<double>& p, int batch, cudaStream_t s)
+void launch_dmma_tile(DmmaTile t, const GemmParams<double>& p, int batch, cudaStream_t s)
 {
     switch(t)
     {
@@ -322,6 +322,12 @@ static void launch_dmma_tile(DmmaTile t, const GemmParams<double>& p, int batch,
     case DmmaTile::t64x64k16:  launch_dmma_cfg<64, 64, 32, 32, 4, KCP, KCQ, 16, 16>(p, batch, s); break;
     }
 }
+
+// instantiated in tile_kernels.cu
+extern template void launch_dmma_tile<false, false>(DmmaTile, const GemmParams<double>&, int, cudaStream_t);
+extern template void launch_dmma_tile<false, true>(DmmaTile, const GemmParams<double>&, int, cudaStream_t);
+extern template void launch_dmma_tile<true, false>(DmmaTile, const GemmParams<double>&, int, cudaStream_t);
+extern template void launch_dmma_tile<true, true>(DmmaTile, const GemmParams<double>&, int, cudaStream_t);
 
 // Tile choice: the largest tile that still gives every SM work.  `full_m` / `full_n` force a
 // tile that spans all M rows (N columns), which the in-place invA application needs.

@@ -273,6 +273,12 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
     if(ws_bytes)
     {
         ws = h->borrow(ws_bytes);
+        if(!ws && use_chain(pr))
+        {
+            // a workspace too small for the flags of narrow strips may hold those of the widest
+            pr.chain_w = 64;
+            ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
+        }
         if(!ws && !have_invA)
         {
             // backup: recursive solve with block-solver leaves needs no workspace
@@ -1623,10 +1629,13 @@ rocblas_status gemm_tiles_impl(rocblas_handle h, rocblas_operation ta, rocblas_o
 struct MixedPlan
 {
     bool   recursive = false;
+    int    chain_w   = 64; // strip width of the chain sub-solves
     size_t inv_bytes = 0, sl_bytes = 0, ch_bytes = 0, total = 0;
 };
 
-MixedPlan mixed_plan(const TrsmProblem<double>& pr, int slices, int moduli)
+// chain_w 0: the width of mixed_chain_width; 64, whose flags take least, where the workspace is
+// too small for that
+MixedPlan mixed_plan(const TrsmProblem<double>& pr, int slices, int moduli, int chain_w = 0)
 {
     MixedPlan p;
     p.recursive = choose_algo(pr) == Algo::recursive;
@@ -1634,7 +1643,8 @@ MixedPlan mixed_plan(const TrsmProblem<double>& pr, int slices, int moduli)
         return p;
     p.inv_bytes = align256((size_t)kInvNB * pr.k() * sizeof(double));
     p.sl_bytes  = mixed_slice_workspace_bytes(pr, slices, moduli);
-    p.ch_bytes  = mixed_chain_workspace_bytes(pr);
+    p.chain_w   = chain_w ? chain_w : mixed_chain_width(pr);
+    p.ch_bytes  = mixed_chain_workspace_bytes(pr, p.chain_w);
     p.total     = p.inv_bytes + align256(p.sl_bytes) + align256(p.ch_bytes);
     return p;
 }
@@ -1662,6 +1672,7 @@ bool mixed_run(TrsmProblem<double> pr, int slices, int moduli, const MixedPlan& 
     rec.moduli   = moduli;
     rec.slice_ws = reinterpret_cast<unsigned char*>(ws) + plan.inv_bytes;
     rec.err_dev  = err;
+    rec.chain_w  = plan.chain_w;
     if(plan.ch_bytes)
         rec.chain_ws = reinterpret_cast<unsigned char*>(ws) + plan.inv_bytes + align256(plan.sl_bytes);
     rec.solve_mixed(0, rec.nblk, 1);
@@ -1710,7 +1721,7 @@ rocblas_status trsm_mixed_impl(rocblas_handle h, rocblas_side side, rocblas_fill
     pr.ldb = ldb;
     pr.stream   = h->stream;
     pr.sm_count = h->sm_count;
-    const MixedPlan plan = mixed_plan(pr, slices, moduli);
+    MixedPlan plan = mixed_plan(pr, slices, moduli);
     if(h->size_query)
         return plan.total ? h->set_optimal_size(plan.total) : rocblas_status_size_unchanged;
     if((st = device_ready(h)) != rocblas_status_success)
@@ -1721,6 +1732,11 @@ rocblas_status trsm_mixed_impl(rocblas_handle h, rocblas_side side, rocblas_fill
         pr.alpha.ptr = alpha;
     int*  err = plan.recursive ? ensure_err(h) : nullptr;
     void* ws  = plan.total ? h->borrow(plan.total) : nullptr;
+    if(plan.recursive && !ws)
+    {
+        plan = mixed_plan(pr, slices, moduli, 64);
+        ws   = h->borrow(plan.total);
+    }
     if(plan.recursive && (!ws || !err))
         return rocblas_status_memory_error;
     if(!mixed_run(pr, slices, moduli, plan, ws, err, true))
@@ -1923,7 +1939,7 @@ rocblas_status trsm_refined_impl(rocblas_handle h, rocblas_side side, rocblas_fi
     // the tested right-hand sides, solved by the plain FP64 form: side left m x c, side right
     // c x n (the same rows of B), ld = their row count.  That solve is a chain of dependent
     // steps whose CTAs hold their SMs while they wait, so it gets a few SMs of its own
-    // (refine_check_sms, chain strips of 32) and the sliced solve's persistent kernels size
+    // (refine_check_sms) and the sliced solve's persistent kernels size
     // their grids for the others.
     TrsmProblem<double> ps = pr;
     const int           srows = left ? m : c, scols = left ? c : n;
@@ -1942,18 +1958,26 @@ rocblas_status trsm_refined_impl(rocblas_handle h, rocblas_side side, rocblas_fi
     const int  nb_flag = (int)ceil_div(left ? m : n, 128);
     // workspace: the precision form's | B0 (m x n) | R (m x n) | the tested right-hand sides |
     // their chain flags | the test's maxima
-    const MixedPlan plan  = mixed_plan(pr, S, moduli);
+    MixedPlan       plan  = mixed_plan(pr, S, moduli);
     const size_t    mn    = (size_t)m * n * sizeof(double);
     const size_t    smp   = (size_t)srows * scols * sizeof(double);
-    // the chain's strip width: 16 wastes half as much DMMA work on up to 8 tested columns
-    const int       ps_w  = tuning().refine_check_w == 16 && c <= 16 ? 16 : 32;
+    // the chain's strip width: that of the up to 8 tested columns, where refine_check_w allows it
+    const int       ps_w  = tuning().refine_check_w == 8 && c <= 8      ? 8
+                            : tuning().refine_check_w == 16 && c <= 16 ? 16
+                                                                       : 32;
     const size_t    fl    = ps_flag    ? (size_t)nb_flag * 2 * sizeof(int)
                             : ps_chain ? chain_workspace_bytes(chain_shape(ps.k(), c, 1, ps_w))
                                        : 0;
-    const size_t    o_b0  = align256(plan.total), o_r = o_b0 + align256(mn);
-    const size_t    o_xs  = o_r + (max_it > 0 ? align256(mn) : 0), o_fl = o_xs + align256(smp);
-    const size_t    o_mx  = o_fl + align256(fl);
-    const size_t    total = o_mx + align256(sizeof(double) * 2 * (size_t)c);
+    size_t o_b0 = 0, o_r = 0, o_xs = 0, o_fl = 0, o_mx = 0, total = 0;
+    auto   lay_out = [&]() {
+        o_b0  = align256(plan.total);
+        o_r   = o_b0 + align256(mn);
+        o_xs  = o_r + (max_it > 0 ? align256(mn) : 0);
+        o_fl  = o_xs + align256(smp);
+        o_mx  = o_fl + align256(fl);
+        total = o_mx + align256(sizeof(double) * 2 * (size_t)c);
+    };
+    lay_out();
     if(h->size_query)
         return h->set_optimal_size(total);
     if((st = device_ready(h)) != rocblas_status_success)
@@ -1967,6 +1991,12 @@ rocblas_status trsm_refined_impl(rocblas_handle h, rocblas_side side, rocblas_fi
         return rocblas_status_internal_error;
     int*           err = ensure_err(h);
     unsigned char* ws  = reinterpret_cast<unsigned char*>(h->borrow(total));
+    if(!ws && plan.recursive)
+    {
+        plan = mixed_plan(pr, S, moduli, 64);
+        lay_out();
+        ws = reinterpret_cast<unsigned char*>(h->borrow(total));
+    }
     if(!ws || !err)
         return rocblas_status_memory_error;
     pr.err_dev = ps.err_dev = err;
@@ -2213,10 +2243,15 @@ rocblas_status trsm_mixed_host_impl(rocblas_handle h, rocblas_side side, rocblas
     const size_t inv_bytes = align256((size_t)kInvNB * k * sizeof(double));
     const size_t sl_bytes  = update_workspace_bytes(std::min(k, DB * kInvNB), n, k, slices, moduli,
                                                     pr.sm_count);
-    const size_t ch_bytes  = mixed_chain_workspace_bytes(pr);
-    const size_t ws_bytes  = inv_bytes + (sl_bytes + 255) / 256 * 256 + (ch_bytes + 255) / 256 * 256;
+    int          chain_w   = mixed_chain_width(pr);
+    const size_t ch_off    = inv_bytes + align256(sl_bytes);
     int*         err       = ensure_err(h);
-    void*        ws        = h->borrow(ws_bytes);
+    void*        ws        = h->borrow(ch_off + align256(mixed_chain_workspace_bytes(pr, chain_w)));
+    if(!ws)
+    {
+        chain_w = 64; // its flags take least
+        ws      = h->borrow(ch_off + align256(mixed_chain_workspace_bytes(pr, chain_w)));
+    }
     if(!ws || !err)
         return rocblas_status_memory_error;
     pr.err_dev = err;
@@ -2230,8 +2265,9 @@ rocblas_status trsm_mixed_host_impl(rocblas_handle h, rocblas_side side, rocblas
     rec.moduli   = moduli;
     rec.slice_ws = reinterpret_cast<unsigned char*>(ws) + inv_bytes;
     rec.err_dev  = err;
-    if(ch_bytes)
-        rec.chain_ws = reinterpret_cast<unsigned char*>(ws) + inv_bytes + (sl_bytes + 255) / 256 * 256;
+    rec.chain_w  = chain_w;
+    if(mixed_chain_workspace_bytes(pr, chain_w))
+        rec.chain_ws = reinterpret_cast<unsigned char*>(ws) + ch_off;
     for(int q = 0; q < nstep && rec.ok; ++q)
     {
         const int d  = forward ? q : nstep - 1 - q;

@@ -573,10 +573,12 @@ static bool sliced_trsm_update(const TrsmProblem<T>& q, int c_lo, int c_hi, int 
     return run_sliced_gemm(g, ws, err, q.stream);
 }
 
-static int mixed_chain_w()
+// Strip width of the precision form's chain sub-solves: that of the largest one on a whole device
+// (the width sizes the workspace, so it must not depend on the SMs that one call leaves to it).
+static int mixed_chain_width(const TrsmProblem<double>& pr)
 {
-    const int t = tuning().chain_w;
-    return t == 32 ? 32 : 64;
+    const int k = std::min<int64_t>((int64_t)tuning().mixed_chain_blocks * kInvNB, pr.k());
+    return chain_width(k, pr.side_left ? pr.n : pr.m, 1, 148);
 }
 
 // ---- precision form of the TRSM ---------------------------------------------------------------
@@ -589,6 +591,7 @@ struct MixedRecursive : Recursive<double>
     void* slice_ws;
     int*  err_dev;
     void* chain_ws = nullptr; // flags of the chain sub-solves (nullptr: recursion to the leaves)
+    int   chain_w  = 64;      // and their strip width
     bool  ok = true;
     // optional hooks around every diagonal-block solve of blocks [b0, b1) (a chain sub-solve or
     // a leaf): the host-buffer path waits for A's data before it and copies the finished rows
@@ -623,7 +626,7 @@ struct MixedRecursive : Recursive<double>
         {
             if(before_diag)
                 before_diag(b0, b1);
-            launch_chain_sub<double>(pr, b0, b1, first, mixed_chain_w(), chain_ws);
+            launch_chain_sub<double>(pr, b0, b1, first, chain_w, chain_ws);
             if(after_diag)
                 after_diag(b0, b1);
             return;
@@ -647,13 +650,13 @@ struct MixedRecursive : Recursive<double>
 };
 
 // Flags of the largest chain sub-solve of the precision form (0: no chain sub-solves).
-static size_t mixed_chain_workspace_bytes(const TrsmProblem<double>& pr)
+static size_t mixed_chain_workspace_bytes(const TrsmProblem<double>& pr, int w)
 {
     const int nbmax = tuning().mixed_chain_blocks;
     if(nbmax < 2)
         return 0;
     const int k = std::min<int64_t>((int64_t)nbmax * kInvNB, pr.k());
-    return chain_workspace_bytes(chain_shape(k, pr.side_left ? pr.n : pr.m, pr.batch, mixed_chain_w()));
+    return chain_workspace_bytes(chain_shape(k, pr.side_left ? pr.n : pr.m, pr.batch, w));
 }
 
 // Largest sliced update of the recursion (the top node's off-diagonal block).

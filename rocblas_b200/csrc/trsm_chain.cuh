@@ -1,6 +1,5 @@
 // Left-looking blocked TRSM in one persistent launch (a dependency chain over the 128-row
-// blocks of the triangle), for few right-hand sides per system and for batches of systems of
-// different sizes.
+// blocks of the triangle), for one system and for batches of systems of different sizes.
 //
 // The reference's left-looking path (special_trsm_template,
 // library/src/blas3/rocblas_trsm_kernels.hpp:1164-1456) walks the diagonal blocks on the
@@ -10,23 +9,36 @@
 //
 //   * work items are (block position j in solve order, system, strip of W right-hand sides),
 //     enumerated level by level: all systems' items of position 0, then of position 1, ...
-//     A CTA claims item ids from a device-side counter in increasing order, so every item an
-//     item depends on (same system and strip, earlier position) was claimed before it by a
-//     CTA that is running; the earliest unfinished claimed item therefore never waits on an
-//     unfinished one: no deadlock, whatever the residency.  With many systems in one launch
-//     (the variable-size batch) a CTA rarely waits at all: the items claimed before it are
-//     mostly other systems' work of the same level;
-//   * an item accumulates M_{b,i} X_i over the finished blocks i in solve order through a
-//     cp.async pipeline of 32- or 16-deep K chunks (ChainCfg) on DMMA (mma.sync m16n8k8 f64),
-//     waiting on a block's flag (ld.acquire.gpu by one thread, then a CTA barrier) before its
-//     first chunk;
-//   * then T = alpha C_b - acc goes to shared memory, X_b = inv(M_bb) T (the caller's or the
-//     fused trtri's invA block, its triangle masked) is written over C_b, and the item's
-//     flag is released (CTA barrier, then st.release.gpu by one thread);
-//   * every wait is bounded (about a second); on timeout the kernel records an error code
-//     and the CTA stops, so a wrong flag cannot hang the GPU.
-// FP32 systems are staged as FP32 and computed in FP64 (the chain is latency-bound, and the
-// DMMA path is the one this kernel has); the result is rounded to FP32 once.
+//     A CTA claims item ids from a device-side counter in increasing order and works them off
+//     in that order, so every item an item depends on (same system and strip, earlier position)
+//     was claimed before it by a CTA that is running; the earliest unfinished claimed item
+//     therefore never waits on an unfinished one: no deadlock, whatever the residency;
+//   * an item computes T = alpha C_b - sum over the finished blocks i of M_{b,i} X_i on DMMA
+//     (mma.sync m16n8k8 f64) from a ring of K chunks in shared memory, then X_b = inv(M_bb) T
+//     (the caller's or the fused trtri's invA block, its triangle masked), written over C_b, and
+//     releases the item's flag (CTA barrier, then st.release.gpu by one thread).
+//
+// The CTA is warp-specialised, because the FP64 tensor pipe (64 FMAs per clock and SM) is what
+// the work is bound by and every instruction that the MMA warps spend on copies is time it
+// idles: 8 warps only read fragments and issue MMAs, 3 warps copy M (and, after an item's last
+// chunk of M, its inverse block) and one warp waits for the flags of the finished blocks
+// (ld.acquire.gpu) and copies X, each through cp.async whose completion arrives on the ring
+// slot's barrier.  The copies of M need no flag, so while the CTA waits for the block before its
+// own (the dependency chain, which is what few right-hand sides are bound by) that block's
+// 128 x 128 tile of M is in shared memory already and one copy of X, two products and one
+// store remain between one flag and the next.  The ring runs on across items: the next item's
+// copies start while the MMA warps finish the current one.
+//
+// Measured (one B200, FP64, against the same chain with copies by the MMA warps and 64-column
+// strips): 3001 x 77 with invA 716 -> 149 us, 8192 x 512 2.31 -> 1.41 ms (24.4 TFLOP/s), 8192 x
+// 8192 23.1 -> 18.0 ms (30.5 TFLOP/s, 0.82 of the tensor pipe's 37.2).  Few right-hand sides are
+// bound by the chain: 5.7 us per block at 8 columns, of which the two products take 1.6 us.
+//
+// Every wait is bounded (ChainParams::wait_cycles, about a second); on timeout the kernel
+// records error code 4, all roles run out without waiting, and the CTA stops, so a wrong flag
+// cannot hang the GPU.
+// FP32 systems are staged as FP32 and computed in FP64 (the DMMA path is the one this kernel
+// has); the result is rounded to FP32 once.
 //
 // The 16 side/uplo/trans/diag cases use the index map of block_solve.cuh: side L solves
 // M Y = alpha C with M = op(A), C = B; side R solves M Y = alpha C with M = op(A)^T, C = B^T;
@@ -35,15 +47,18 @@
 // Unit diagonals need nothing here: invA already holds the inverse of the unit triangle.
 #pragma once
 #include "gemm_dmma.cuh"
+#include "mbarrier.cuh"
 #include "timing.hpp"
 
 namespace rb200
 {
 
-constexpr int kChainThreads = 256;
-constexpr int kChainBK      = 16;
-constexpr int kChainStages  = 4;
-constexpr int kChainNB      = 128;
+constexpr int kChainMmaWarps  = 8;
+constexpr int kChainCopyWarps = 3; // copies of M and of the inverse blocks
+constexpr int kChainMmaThreads  = 32 * kChainMmaWarps;
+constexpr int kChainCopyThreads = 32 * kChainCopyWarps;
+constexpr int kChainThreads   = kChainMmaThreads + kChainCopyThreads + 32; // + the X warp
+constexpr int kChainNB        = 128;
 
 // One system of a variable-size chain launch (sorted by block count, largest first).
 template <typename T>
@@ -109,90 +124,150 @@ __device__ __forceinline__ void chain_st_release(int* p, int v)
 }
 
 template <typename T>
-__device__ __forceinline__ void chain_cp_async(T* smem, const T* gmem, bool valid)
+__device__ __forceinline__ void chain_cp_async(uint32_t smem, const T* gmem, bool valid)
 {
-    const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-    const int      n = valid ? (int)sizeof(T) : 0;
+    const int n = valid ? (int)sizeof(T) : 0;
     if constexpr(sizeof(T) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem), "r"(n) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem), "l"(gmem), "r"(n) : "memory");
     else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(s), "l"(gmem), "r"(n) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem), "l"(gmem), "r"(n) : "memory");
 }
 
-// smem layouts: P (M rows o x K) [k][o] pitch 132 (KCP = false) or [o][k] pitch BK+4 (KCP);
-// Q (K x W) [k][n] pitch W+4 (KCQ = false) or [n][k] pitch BK+4 (KCQ); elements of type T.
-// K chunks are 32 deep in 3 stages where that fits in shared memory (fewer CTA barriers per
-// MMA; measured faster for one large system), else 16 deep in 4 stages (measured faster for
-// the variable-size batch, VB); either depth divides the 128-row blocks, so a chunk never
-// spans two blocks.
-template <typename T, int W, bool KCP, bool KCQ, bool VB = false>
+// Shared memory: a ring of stages, each a chunk of M (128 rows o x kBK columns k) and of X (kBK x
+// W), then the tile T (128 x W doubles).  Layouts: M [k][o] (KCP = false) or [o][k] (KCP), X
+// [k][n] (KCQ = false) or [n][k] (KCQ), elements of type T.  Row pitches keep the fragment reads
+// (lanes (g, t) reading element (g, t) or (t, g)) free of bank conflicts: for doubles 4 or 12 mod
+// 16 (two half-warp phases), for floats 8 mod 32 where t is the slow index and 4 mod 32 where g is.
+// Chunks are 32 deep where four stages fit in shared memory (narrow strips, whose wait for a block
+// is covered by the whole tile of M and the start of the inverse in the ring), else 16 deep;
+// either depth divides the 128-row blocks, so a chunk never spans two blocks.
+template <typename T, int W, bool KCP, bool KCQ>
 struct ChainCfg
 {
-    static constexpr size_t bytes(int bk, int stages)
+    static constexpr int slow_pitch(int n) { return sizeof(T) == 8 ? n + 4 : n + (n % 32 == 0 || n % 32 == 16 ? 8 : 0); }
+    static constexpr int pitch_p(int bk) { return KCP ? bk + 4 : slow_pitch(kChainNB); }
+    static constexpr int pitch_q(int bk) { return KCQ ? bk + 4 : slow_pitch(W); }
+    static constexpr int stage_p(int bk) { return KCP ? kChainNB * pitch_p(bk) : bk * pitch_p(bk); }
+    static constexpr int stage_q(int bk) { return KCQ ? W * pitch_q(bk) : bk * pitch_q(bk); }
+    static constexpr size_t kBytesT = sizeof(double) * (size_t)kChainNB * (W + 4);
+    static constexpr size_t kRoom   = 226 * 1024 - kBytesT; // for the ring; the barriers take the rest
+    static constexpr int stages(int bk)
     {
-        const int pp = KCP ? bk + 4 : kChainNB + 4, pq = KCQ ? bk + 4 : W + 4;
-        const int sp = KCP ? kChainNB * pp : bk * pp, sq = KCQ ? W * pq : bk * pq;
-        return sizeof(T) * (size_t)stages * (sp + sq) + sizeof(double) * (size_t)kChainNB * (W + 4);
+        return (int)(kRoom / (sizeof(T) * (size_t)(stage_p(bk) + stage_q(bk))));
     }
-    static constexpr bool kDeep   = !VB && bytes(32, 3) <= 227 * 1024 - 64; // room for the static words
-    static constexpr int kBK      = kDeep ? 32 : kChainBK;
-    static constexpr int kStages  = kDeep ? 3 : kChainStages;
-    static constexpr int kPitchP  = KCP ? kBK + 4 : kChainNB + 4;
-    static constexpr int kPitchQ  = KCQ ? kBK + 4 : W + 4;
-    static constexpr int kStageP  = KCP ? kChainNB * kPitchP : kBK * kPitchP;
-    static constexpr int kStageQ  = KCQ ? W * kPitchQ : kBK * kPitchQ;
+    static constexpr int kBK      = stages(32) >= 4 ? 32 : 16;
+    static constexpr int kStages  = stages(kBK) < 8 ? stages(kBK) : 8;
+    static constexpr int kPitchP  = pitch_p(kBK);
+    static constexpr int kPitchQ  = pitch_q(kBK);
+    static constexpr int kStageP  = stage_p(kBK);
+    static constexpr int kStageQ  = stage_q(kBK);
     static constexpr int kStage   = kStageP + kStageQ; // elements of T
     static constexpr int kPitchT  = W + 4;             // T tile [k = row o][n], doubles
-    static constexpr size_t kSmem = bytes(kBK, kStages);
+    static constexpr size_t kRing = sizeof(T) * (size_t)kStages * kStage;
+    static constexpr size_t kSmem = kRing + kBytesT;
+    static_assert(kStages >= 3 && kRing % 16 == 0, "ring");
+    // MMA warps: 32 x 32 blocks of the 128 x 64 item, or 16 rows x all W columns of a narrower one
+    // (narrower warp rows make the two products of an item equally long for every warp)
+    static constexpr int kWarpsN = W == 64 ? 2 : 1;
+    static constexpr int kWM     = kChainNB * kWarpsN / kChainMmaWarps; // rows of a warp
+    static constexpr int kWN     = W / kWarpsN;                         // columns of a warp
+    static constexpr int TM = kWM / 16, TN = kWN / 8;
+    // independent accumulators per output tile, so that a warp's MMAs do not wait on one another
+    static constexpr int kSplit = TM * TN == 1 ? 4 : TM * TN == 2 ? 2 : 1;
 };
 
-// W right-hand sides per item (32 or 64); 8 warps as 4 (rows) x 2 (columns), each warp
-// 32 x W/2 of the 128 x W block.  KCP: M's K index is contiguous in memory (tM); KCQ: C's
-// row index is contiguous (side L).  VB: the variable-size tables of p describe the items.
+// One claimed item, resolved for all roles.
+template <typename T>
+struct ChainItem
+{
+    const T* M;     // M(r0, 0) in A's storage
+    const T* inv;   // the block's inverse
+    T*       C;     // C(0, c0) in B's storage
+    int64_t  lda, ldb;
+    int64_t  item;  // < 0: no more items
+    int*     flag0; // flag of solve position jj: flag0 + (VB ? vL[jj] : jj * fstride)
+    int64_t  fstride;
+    int      r0, bs, wv, nb, forward;
+    int      klo, khi, ktop; // rows of the finished blocks [klo, khi), chunks counted from ktop when backward
+    int      nk, nki;        // chunks of M and of the inverse
+};
+
+// W right-hand sides per item (8, 16, 32 or 64).  KCP: M's K index is contiguous in memory (tM);
+// KCQ: C's row index is contiguous (side L).  VB: the variable-size tables of p describe the items.
 template <typename T, int W, bool KCP, bool KCQ, bool VB>
 __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParams<T> p)
 {
-    using Cfg = ChainCfg<T, W, KCP, KCQ, VB>;
-    constexpr int TM = 2, TN = W / 16; // per warp: 32 rows x W/2 columns
-    constexpr int WN = W / 2;
+    using Cfg = ChainCfg<T, W, KCP, KCQ>;
+    constexpr int TM = Cfg::TM, TN = Cfg::TN, BK = Cfg::kBK, NS = Cfg::kStages, SP = Cfg::kSplit;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T*         smem = reinterpret_cast<T*>(smem_raw);
-    double*    Ts   = reinterpret_cast<double*>(smem_raw + sizeof(T) * (size_t)Cfg::kStages * Cfg::kStage);
-    __shared__ int64_t s_item;
-    __shared__ int     s_abort;
+    T*      ring = reinterpret_cast<T*>(smem_raw);
+    double* Ts   = reinterpret_cast<double*>(smem_raw + Cfg::kRing);
+    __shared__ ChainItem<T> s_item[2];
+    __shared__ uint64_t     full[NS], empty[NS], item_full[2], item_empty[2];
+    __shared__ int          s_abort;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp & 3, wn = warp >> 2;
-    const int g = lane >> 2, t = lane & 3;
+    if(tid == 0)
+    {
+        s_abort = 0;
+        for(int i = 0; i < NS; ++i)
+        {
+            mbar_init(&full[i], kChainCopyThreads + 32);
+            mbar_init(&empty[i], kChainMmaWarps);
+        }
+        for(int i = 0; i < 2; ++i)
+        {
+            mbar_init(&item_full[i], 1);
+            mbar_init(&item_empty[i], kChainThreads / 32);
+        }
+    }
+    __syncthreads();
+
+    // Bounded waits.  A barrier's owner may itself be waiting for a flag, so barriers wait longer;
+    // once a wait ran out (s_abort) every other one returns at once.
+    auto aborted = [&]() { return *(volatile int*)&s_abort != 0; };
+    auto give_up = [&]() {
+        atomicExch(p.error, 4);
+        *(volatile int*)&s_abort = 1;
+    };
+    auto wait_bar = [&](uint64_t* bar, uint32_t parity) {
+        if(mbar_try_wait(bar, parity))
+            return;
+        const long long t0 = clock64();
+        while(!mbar_try_wait(bar, parity))
+        {
+            if(aborted())
+                return;
+            if(clock64() - t0 > 4 * p.wait_cycles + (1ll << 24))
+            {
+                give_up();
+                return;
+            }
+        }
+    };
+
     // alpha == 0 anywhere in the call means B := 0 with A unreferenced, also for sub-solves
     // that would otherwise apply 1
     const double ua    = (double)p.alpha.get();
     const double alpha = ua == 0.0 ? 0.0 : (p.first ? ua : 1.0);
-    ChainVbHeader<T> H{};
-    if constexpr(VB)
-        H = *p.vhdr;
-    int* const    flags = VB ? H.flags : p.flags;
-    const int64_t total = VB ? (H.maxnb > 0 ? H.vL[H.maxnb] : 0) : p.items;
+    const bool   zero  = alpha == 0.0;
 
-    if(tid == 0)
-        s_abort = 0;
-
-    for(;;)
-    {
-        __syncthreads();
-        if(tid == 0)
-            s_item = atomicAdd(reinterpret_cast<unsigned long long*>(p.counter), 1ull);
-        __syncthreads();
-        const int64_t item = s_item;
-        if(item >= total || s_abort)
-            break;
-
-        // ---- resolve the item: (level j, system, strip) ------------------------------------
+    // claim the next item (one thread)
+    auto claim = [&](ChainItem<T>& q) {
+        ChainVbHeader<T> H{};
+        if constexpr(VB)
+            H = *p.vhdr;
+        const int64_t total = VB ? (H.maxnb > 0 ? H.vL[H.maxnb] : 0) : p.items;
+        const int64_t item  = aborted() ? total
+                                        : (int64_t)atomicAdd(reinterpret_cast<unsigned long long*>(p.counter), 1ull);
+        if(item >= total)
+        {
+            q.item = -1;
+            return;
+        }
+        int      k, ncols, j, strip;
         const T* A;
-        const T* invA;
         T*       B;
-        int64_t  lda, ldb, sysi;
-        int      k, ncols, nb, ns, forward, j, strip;
         if constexpr(VB)
         {
             // level: last j with vL[j] <= item; system: last i < vcnt[j] with vP[i] <= r
@@ -216,290 +291,478 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                 else
                     z = mid - 1;
             }
-            sysi  = a;
             strip = r - H.vP[a];
-            const ChainSys<T> q = H.vsys[a];
-            A = q.A; invA = q.invA; B = q.B; lda = q.lda; ldb = q.ldb;
-            k = q.k; ncols = q.ncols; nb = q.nb; ns = q.ns; forward = q.forward;
+            const ChainSys<T> v = H.vsys[a];
+            A = v.A; q.inv = v.invA; B = v.B; q.lda = v.lda; q.ldb = v.ldb;
+            k = v.k; ncols = v.ncols; q.nb = v.nb; q.forward = v.forward;
+            q.flag0   = H.flags + H.vP[a] + strip;
+            q.fstride = 0;
         }
         else
         {
             strip = (int)(item % p.ns);
-            const int64_t js = item / p.ns;
-            sysi  = js % p.systems;
-            j     = (int)(js / p.systems);
-            A = p.A.get((int)sysi); invA = p.invA.get((int)sysi); B = p.B.get((int)sysi);
-            lda = p.lda; ldb = p.ldb; k = p.k; ncols = p.ncols; nb = p.nb; ns = p.ns;
-            forward = p.forward;
+            const int64_t js   = item / p.ns;
+            const int     sysi = (int)(js % p.systems);
+            j = (int)(js / p.systems);
+            A = p.A.get(sysi); q.inv = p.invA.get(sysi); B = p.B.get(sysi);
+            q.lda = p.lda; q.ldb = p.ldb; k = p.k; ncols = p.ncols; q.nb = p.nb;
+            q.forward = p.forward;
+            q.flag0   = p.flags + (int64_t)sysi * p.ns + strip;
+            q.fstride = (int64_t)p.systems * p.ns;
         }
-        // flag of this system's strip at solve position jj (= that item's id)
-        auto flag_of = [&](int jj) -> int* {
-            if constexpr(VB)
-                return flags + H.vL[jj] + H.vP[sysi] + strip;
+        const int b = q.forward ? j : q.nb - 1 - j;
+        q.item = item;
+        q.r0   = b * kChainNB;
+        q.bs   = min(kChainNB, k - q.r0);
+        q.wv   = min(W, ncols - strip * W);
+        q.M    = KCP ? A + (int64_t)q.r0 * q.lda : A + q.r0;
+        q.inv += (int64_t)b * kChainNB * kChainNB;
+        q.C    = KCQ ? B + (int64_t)strip * W * q.ldb : B + strip * W;
+        // K rows of the finished blocks: forward [0, r0) ascending; backward [r0 + bs, k)
+        // descending, in chunks of BK rows aligned to multiples of BK (never across a block)
+        q.klo  = q.forward ? 0 : q.r0 + q.bs;
+        q.khi  = q.forward ? q.r0 : k;
+        q.ktop = (int)ceil_div(q.khi, BK) * BK;
+        q.nk   = zero ? 0 : q.forward ? q.ktop / BK : (q.ktop - q.klo) / BK;
+        q.nki  = zero ? 0 : (int)ceil_div(q.bs, BK);
+    };
+    // barrier of the MMA warps; true in all of them if any saw a wait run out, so that they leave
+    // the item loop together
+    auto mma_sync_stop = [&]() -> bool {
+        int any;
+        asm volatile("{\n\t.reg .pred p, q;\n\t"
+                     "setp.ne.s32 p, %1, 0;\n\t"
+                     "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
+                     "selp.s32 %0, 1, 0, q;\n\t}"
+                     : "=r"(any)
+                     : "r"((int)aborted()), "n"(kChainMmaThreads)
+                     : "memory");
+        return any != 0;
+    };
+    auto item_done = [&](int n) {
+        __syncwarp();
+        if(lane == 0)
+            mbar_arrive(&item_empty[n & 1]);
+    };
+
+    if(warp >= kChainMmaWarps)
+    {
+        const bool  copies_m = warp < kChainMmaWarps + kChainCopyWarps;
+        uint32_t    st = 0, ph = 1; // ring slot, parity of its last release
+        ChainItem<T> q;
+        auto slot = [&]() { wait_bar(&empty[st], ph); };
+        auto advance = [&]() {
+            if(++st == NS)
+            {
+                st = 0;
+                ph ^= 1;
+            }
+        };
+        for(int n = 0;; ++n)
+        {
+            if(warp == kChainMmaWarps && lane == 0)
+            {
+                if(n >= 2)
+                    wait_bar(&item_empty[n & 1], ((n >> 1) - 1) & 1);
+                claim(s_item[n & 1]);
+                mbar_arrive(&item_full[n & 1]);
+            }
+            __syncwarp();
+            wait_bar(&item_full[n & 1], (n >> 1) & 1);
+            if(aborted())
+                break;
+            q = s_item[n & 1];
+            if(q.item < 0)
+                break;
+            if(copies_m)
+            {
+                // ---- chunks of M, then of the inverse --------------------
+                // A warp copies every third line of a chunk: a K column (128 rows; four copies
+                // per lane) or, K contiguous, 32 / BK rows of BK columns.
+                constexpr int kLines = KCP ? kChainNB * BK / 32 : BK;
+                constexpr int kPer   = KCP ? 1 : kChainNB / 32; // copies per lane and line
+                const int     cw  = warp - kChainMmaWarps;
+                const int     o0  = KCP ? lane / BK : lane, kk0 = KCP ? lane % BK : 0;
+                constexpr int kLineO = KCP ? 32 / BK : 0, kLineK = KCP ? 0 : 1;
+                constexpr uint32_t kDstLine = (uint32_t)sizeof(T) * (KCP ? kLineO : 1) * Cfg::kPitchP;
+                const uint32_t dst0 = smem_u32(ring) + (uint32_t)sizeof(T) * (KCP ? o0 * Cfg::kPitchP + kk0 : o0)
+                                      + cw * kDstLine;
+                const int64_t line = KCP ? kLineO * q.lda : q.lda;
+                for(int i = 0; i < q.nk; ++i)
+                {
+                    const int k0 = q.forward ? i * BK : q.ktop - (i + 1) * BK;
+                    slot();
+                    uint32_t dst = dst0 + st * (uint32_t)(sizeof(T) * Cfg::kStage);
+                    const T* src = (KCP ? q.M + (k0 + kk0) + (int64_t)o0 * q.lda : q.M + o0 + (int64_t)k0 * q.lda)
+                                   + cw * line;
+                    const bool whole = q.bs == kChainNB && k0 + BK <= q.khi;
+                    if(whole)
+                    {
+#pragma unroll 4
+                        for(int e = cw; e < kLines; e += kChainCopyWarps)
+                        {
+#pragma unroll
+                            for(int u = 0; u < kPer; ++u)
+                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), src + u * 32, true);
+                            dst += kChainCopyWarps * kDstLine;
+                            src += kChainCopyWarps * line;
+                        }
+                    }
+                    else
+                    {
+#pragma unroll 1
+                        for(int e = cw; e < kLines; e += kChainCopyWarps)
+                        {
+#pragma unroll
+                            for(int u = 0; u < kPer; ++u)
+                            {
+                                const bool valid = o0 + e * kLineO + u * 32 < q.bs && k0 + kk0 + e * kLineK < q.khi;
+                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), valid ? src + u * 32 : q.M, valid);
+                            }
+                            dst += kChainCopyWarps * kDstLine;
+                            src += kChainCopyWarps * line;
+                        }
+                    }
+                    mbar_arrive_cp_async(&full[st]);
+                    advance();
+                }
+                // inv(M_bb)(o, k) = tM ? invA(k, o) : invA(o, k); rows and columns >= bs are zero (the
+                // opposite triangle, which a caller's invA may leave undefined, is masked where the
+                // fragments are read)
+                for(int i = 0; i < q.nki; ++i)
+                {
+                    const int k0 = i * BK;
+                    slot();
+                    uint32_t dst = dst0 + st * (uint32_t)(sizeof(T) * Cfg::kStage);
+                    if(q.bs == kChainNB)
+                    {
+                        constexpr int kLine = (KCP ? kLineO : 1) * kChainNB;
+                        const T* src = (KCP ? q.inv + (k0 + kk0) + o0 * kChainNB : q.inv + o0 + k0 * kChainNB) + cw * kLine;
+#pragma unroll 4
+                        for(int e = cw; e < kLines; e += kChainCopyWarps)
+                        {
+#pragma unroll
+                            for(int u = 0; u < kPer; ++u)
+                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), src + u * 32, true);
+                            dst += kChainCopyWarps * kDstLine;
+                            src += kChainCopyWarps * kLine;
+                        }
+                    }
+                    else
+#pragma unroll 2
+                    for(int e = cw; e < kLines; e += kChainCopyWarps)
+                    {
+#pragma unroll
+                        for(int u = 0; u < kPer; ++u)
+                        {
+                            const int  o = o0 + e * kLineO + u * 32, kr = k0 + kk0 + e * kLineK;
+                            const bool valid = o < q.bs && kr < q.bs;
+                            chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T),
+                                              valid ? q.inv + (KCP ? kr + o * kChainNB : o + kr * kChainNB) : q.inv, valid);
+                        }
+                        dst += kChainCopyWarps * kDstLine;
+                    }
+                    mbar_arrive_cp_async(&full[st]);
+                    advance();
+                }
+            }
             else
-                return flags + ((int64_t)jj * p.systems + sysi) * ns + strip;
-        };
-        const int b  = forward ? j : nb - 1 - j;
-        const int r0 = b * kChainNB;
-        const int bs = min(kChainNB, k - r0);
-        const int c0 = strip * W;
-        const int wv = min(W, ncols - c0);
-        const T*  inv = invA + (int64_t)b * kChainNB * kChainNB;
+            {
+                // ---- chunks of X, each block's after its flag; nothing beside the inverse --------
+                constexpr int kFast = KCQ ? BK : W; // lanes run along this dimension
+                constexpr int kLanes = kFast < 32 ? kFast : 32;
+                constexpr int kStep = 32 / kLanes;  // lines (of the other dimension) per warp copy
+                constexpr int kRep  = kFast / kLanes;
+                constexpr int kLines = W * BK / kFast;
+                const int     f0 = lane % kLanes, l0 = lane / kLanes;
+                const uint32_t dst0 = smem_u32(ring)
+                                      + (uint32_t)sizeof(T) * (Cfg::kStageP + l0 * Cfg::kPitchQ + f0);
+                const T* const src0 = q.C + f0 + l0 * q.ldb;
+                const int64_t  line = kStep * q.ldb;
+                constexpr uint32_t kDstLine = (uint32_t)sizeof(T) * kStep * Cfg::kPitchQ;
+                // solve positions [0, done) of the item's nprev earlier ones are known finished; one
+                // round of loads looks at the next 32 flags, so finished blocks cost no round trip each
+                const int nprev = q.forward ? q.r0 / kChainNB : q.nb - 1 - q.r0 / kChainNB;
+                int       done  = 0;
+                for(int i = 0; i < q.nk; ++i)
+                {
+                    const int k0  = q.forward ? i * BK : q.ktop - (i + 1) * BK;
+                    const int pos = q.forward ? k0 / kChainNB : q.nb - 1 - k0 / kChainNB;
+                    slot();
+                    if(pos >= done)
+                    {
+                        const long long t0 = clock64();
+                        for(;;)
+                        {
+                            const int jj = done + lane;
+                            int       f  = 0;
+                            if(jj < nprev)
+                            {
+                                if constexpr(VB)
+                                    f = chain_ld_acquire(q.flag0 + p.vhdr->vL[jj]);
+                                else
+                                    f = chain_ld_acquire(q.flag0 + jj * q.fstride);
+                            }
+                            const unsigned ready = __ballot_sync(0xffffffffu, f != 0);
+                            done += ready == 0xffffffffu ? 32 : __ffs(~ready) - 1;
+                            if(pos < done || __any_sync(0xffffffffu, aborted()))
+                                break;
+                            if(__any_sync(0xffffffffu, clock64() - t0 > p.wait_cycles))
+                            {
+                                if(lane == 0)
+                                    give_up();
+                                break;
+                            }
+                        }
+                        __syncwarp(); // the lanes' acquires order the warp's copies of X below
+                    }
+                    uint32_t dst = dst0 + st * (uint32_t)(sizeof(T) * Cfg::kStage);
+                    const T* src = src0 + (KCQ ? k0 : k0 * q.ldb);
+                    if(q.wv == W && k0 + BK <= q.khi)
+                    {
+#pragma unroll 8
+                        for(int e = 0; e < kLines; e += kStep, src += line, dst += kDstLine)
+#pragma unroll
+                            for(int u = 0; u < kRep; ++u)
+                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), src + u * 32, true);
+                    }
+                    else
+                    {
+#pragma unroll 1
+                        for(int e = 0; e < kLines; e += kStep, src += line, dst += kDstLine)
+#pragma unroll
+                            for(int u = 0; u < kRep; ++u)
+                            {
+                                const int  f = f0 + u * 32, l = l0 + e;
+                                const bool valid = (KCQ ? l : f) < q.wv && k0 + (KCQ ? f : l) < q.khi;
+                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), valid ? src + u * 32 : q.C, valid);
+                            }
+                    }
+                    mbar_arrive_cp_async(&full[st]);
+                    advance();
+                }
+                for(int i = 0; i < q.nki; ++i)
+                {
+                    slot();
+                    mbar_arrive(&full[st]); // its share of the slot's arrivals
+                    advance();
+                }
+            }
+            item_done(n);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
+    }
 
-        // M(r, c) and C(r, col) addresses
-        auto maddr = [&](int rr, int cc) -> const T* {
-            return KCP ? A + cc + (int64_t)rr * lda : A + rr + (int64_t)cc * lda;
-        };
-        auto caddr = [&](int rr, int col) -> T* {
-            return KCQ ? B + rr + (int64_t)col * ldb : B + col + (int64_t)rr * ldb;
-        };
-
-        double acc[TM][TN][4];
+    // ---- the MMA warps -----------------------------------------------------------------------
+    // Warps 4..7 take the block rows in opposite order, so that the two warps of a scheduler
+    // share the triangle of the inverse evenly.
+    const int g = lane >> 2, t = lane & 3;
+    const int wn  = Cfg::kWarpsN == 2 ? warp >> 2 : 0;
+    const int wm  = warp < 4 ? warp : Cfg::kWarpsN == 2 ? 7 - warp : 11 - warp;
+    const int row0 = wm * Cfg::kWM, col0 = wn * Cfg::kWN;
+    uint32_t  st = 0, ph = 0;
+    auto advance = [&]() {
+        __syncwarp();
+        if(lane == 0)
+            mbar_arrive(&empty[st]);
+        if(++st == NS)
+        {
+            st = 0;
+            ph ^= 1;
+        }
+    };
+    auto ldP = [&](const T* sP, int o, int kk) -> double {
+        return (double)(KCP ? sP[o * Cfg::kPitchP + kk] : sP[kk * Cfg::kPitchP + o]);
+    };
+    auto ldQ = [&](const T* sQ, int n, int kk) -> double {
+        return (double)(KCQ ? sQ[n * Cfg::kPitchQ + kk] : sQ[kk * Cfg::kPitchQ + n]);
+    };
+    auto load_a = [&](double (&fa)[TM][4], const T* sP, int kk) {
 #pragma unroll
         for(int i = 0; i < TM; ++i)
+        {
+            const int o = row0 + i * 16 + g;
+            fa[i][0] = ldP(sP, o, kk);
+            fa[i][1] = ldP(sP, o + 8, kk);
+            fa[i][2] = ldP(sP, o, kk + 4);
+            fa[i][3] = ldP(sP, o + 8, kk + 4);
+        }
+    };
+
+    for(int n = 0;; ++n)
+    {
+        wait_bar(&item_full[n & 1], (n >> 1) & 1);
+        if(mma_sync_stop())
+            break;
+        const ChainItem<T> q = s_item[n & 1];
+        if(q.item < 0)
+            break;
+        // C(r0 + o, col) of this thread's output (i, jn, e)
+        auto caddr = [&](int o, int col) -> T* {
+            return KCQ ? q.C + (q.r0 + o) + (int64_t)col * q.ldb : q.C + col + (int64_t)(q.r0 + o) * q.ldb;
+        };
+        auto out_o = [&](int i, int e) { return row0 + i * 16 + g + (e >> 1) * 8; };
+        auto out_n = [&](int jn, int e) { return col0 + jn * 8 + 2 * t + (e & 1); };
+
+        // ---- 1. acc = M[rows of b, finished rows] X[finished rows, strip] -------------------
+        // The sum starts at zero and meets C_b once (C_b in the accumulator would round every
+        // small term at C_b's magnitude).  Narrow strips read C_b before the chunks arrive (no
+        // other item writes it); wide ones, whose registers are full, after the products.
+        constexpr bool kEarlyC = W <= 16;
+        auto read_c = [&](double (&c)[TN][4], int i) {
 #pragma unroll
             for(int jn = 0; jn < TN; ++jn)
 #pragma unroll
                 for(int e = 0; e < 4; ++e)
-                    acc[i][jn][e] = 0.0;
-
-        // ---- 1. acc = M[rows of b, finished rows] * X[finished rows, strip] ---------------
-        // K rows of the finished blocks: forward [0, r0) ascending; backward [r0 + bs, k)
-        // descending, in chunks of Cfg::kBK rows aligned to multiples of kBK (never across a
-        // block).
-        const int klo  = forward ? 0 : r0 + bs;
-        const int khi  = forward ? r0 : k;
-        const int ktop = (int)ceil_div(khi, Cfg::kBK) * Cfg::kBK;
-        const int nk   = forward ? (int)ceil_div(khi, Cfg::kBK) : (ktop - klo) / Cfg::kBK;
-        const bool zero = alpha == 0.0;
-        int waited = forward ? 0 : nb; // blocks known finished: [0, waited) or [waited, nb)
-
-        auto chunk_row0 = [&](int c) { return forward ? c * Cfg::kBK : ktop - (c + 1) * Cfg::kBK; };
-        // wait until the block holding chunk c is finished (uniform across the CTA)
-        auto wait_chunk = [&](int c) -> bool {
-            const int  blk  = max(chunk_row0(c), klo) / kChainNB;
-            const bool need = forward ? blk >= waited : blk < waited;
-            if(!need)
-                return true;
-            if(tid == 0)
-            {
-                const int*      f  = flag_of(forward ? blk : nb - 1 - blk);
-                const long long t0 = clock64();
-                while(chain_ld_acquire(f) == 0)
                 {
-                    if(clock64() - t0 > p.wait_cycles)
-                    {
-                        atomicExch(p.error, 4);
-                        s_abort = 1;
-                        break;
-                    }
+                    const int o = out_o(i, e), col = out_n(jn, e);
+                    c[jn][e] = !zero && o < q.bs && col < q.wv ? alpha * (double)__ldcg(caddr(o, col)) : 0.0;
                 }
-            }
-            __syncthreads();
-            if(s_abort)
-                return false;
-            waited = forward ? blk + 1 : blk;
-            return true;
         };
-        auto load_chunk = [&](int stage, int c) {
-            T*        sP = smem + stage * Cfg::kStage;
-            T*        sQ = sP + Cfg::kStageP;
-            const int k0 = chunk_row0(c);
-            // P: M(r0 + o, k0 + kk), o < 128, kk < 16
+        double acc[SP][TM][TN][4], cv[TM][TN][4];
+        if constexpr(kEarlyC)
 #pragma unroll
-            for(int i = 0; i < kChainNB * Cfg::kBK / kChainThreads; ++i)
-            {
-                const int e = tid + i * kChainThreads;
-                int       o, kk;
-                if(KCP) { kk = e % Cfg::kBK; o = e / Cfg::kBK; }
-                else    { o = e % kChainNB; kk = e / kChainNB; }
-                const int  kr    = k0 + kk;
-                const bool valid = o < bs && kr >= klo && kr < khi;
-                const T*   src   = valid ? maddr(r0 + o, kr) : A;
-                T*         dst   = KCP ? sP + o * Cfg::kPitchP + kk : sP + kk * Cfg::kPitchP + o;
-                chain_cp_async<T>(dst, src, valid);
-            }
-            // Q: C(k0 + kk, c0 + n), kk < 16, n < W
+            for(int i = 0; i < TM; ++i)
+                read_c(cv[i], i);
 #pragma unroll
-            for(int i = 0; i < W * Cfg::kBK / kChainThreads; ++i)
-            {
-                const int e = tid + i * kChainThreads;
-                int       n, kk;
-                if(KCQ) { kk = e % Cfg::kBK; n = e / Cfg::kBK; }
-                else    { n = e % W; kk = e / W; }
-                const int  kr    = k0 + kk;
-                const bool valid = n < wv && kr >= klo && kr < khi;
-                const T*   src   = valid ? caddr(kr, c0 + n) : B;
-                T*         dst   = KCQ ? sQ + n * Cfg::kPitchQ + kk : sQ + kk * Cfg::kPitchQ + n;
-                chain_cp_async<T>(dst, src, valid);
-            }
-        };
-        auto ldP = [&](const T* sP, int o, int kk) -> double {
-            return (double)(KCP ? sP[o * Cfg::kPitchP + kk] : sP[kk * Cfg::kPitchP + o]);
-        };
-        auto ldQ = [&](const T* sQ, int n, int kk) -> double {
-            return (double)(KCQ ? sQ[n * Cfg::kPitchQ + kk] : sQ[kk * Cfg::kPitchQ + n]);
-        };
-
-        if(!zero && nk > 0)
+        for(int s = 0; s < SP; ++s)
+#pragma unroll
+            for(int i = 0; i < TM; ++i)
+#pragma unroll
+                for(int jn = 0; jn < TN; ++jn)
+#pragma unroll
+                    for(int e = 0; e < 4; ++e)
+                        acc[s][i][jn][e] = 0.0;
+        // Fragments are read one k step ahead of the MMAs that use them, for wide strips also
+        // across chunks (a narrow one must not hold back a step of the chunk that is there for
+        // the next, whose block of X may be microseconds away).
         {
-            bool ok = true;
-#pragma unroll 1
-            for(int s = 0; s < Cfg::kStages - 1; ++s)
-            {
-                if(s < nk && ok)
+            double fa[2][TM][4], fb[2][TN][2];
+            auto   read = [&](int f, int ks) {
+                const T*  sP = ring + st * Cfg::kStage;
+                const T*  sQ = sP + Cfg::kStageP;
+                const int kk = ks * 8 + t;
+                load_a(fa[f], sP, kk);
+#pragma unroll
+                for(int jn = 0; jn < TN; ++jn)
                 {
-                    ok = wait_chunk(s);
-                    if(ok)
-                        load_chunk(s, s);
+                    const int nn = col0 + jn * 8 + g;
+                    fb[f][jn][0] = ldQ(sQ, nn, kk);
+                    fb[f][jn][1] = ldQ(sQ, nn, kk + 4);
                 }
-                cp_async_commit();
+            };
+            auto wait_full = [&]() { wait_bar(&full[st], ph); };
+            constexpr bool kAcross = W >= 32;
+            constexpr int  KS      = BK / 8;
+            static_assert(KS % 2 == 0, "the fragment buffers alternate");
+            if(kAcross && q.nk > 0)
+            {
+                wait_full();
+                read(0, 0);
             }
 #pragma unroll 1
-            for(int kt = 0; kt < nk && ok; ++kt)
+            for(int c = 0; c < q.nk; ++c)
             {
-                cp_async_wait<Cfg::kStages - 2>();
-                __syncthreads();
-                const T* sP = smem + (kt % Cfg::kStages) * Cfg::kStage;
-                const T* sQ = sP + Cfg::kStageP;
-#pragma unroll
-                for(int ks = 0; ks < Cfg::kBK / 8; ++ks)
+                if(!kAcross)
                 {
-                    const int kk = ks * 8 + t;
-                    double    fa[TM][4], fb[TN][2];
+                    wait_full();
+                    read(0, 0);
+                }
 #pragma unroll
-                    for(int i = 0; i < TM; ++i)
+                for(int ks = 0; ks < KS; ++ks)
+                {
+                    if(ks + 1 < KS)
+                        read((ks + 1) & 1, ks + 1);
+                    else
                     {
-                        const int o = wm * 32 + i * 16 + g;
-                        fa[i][0] = ldP(sP, o, kk);
-                        fa[i][1] = ldP(sP, o + 8, kk);
-                        fa[i][2] = ldP(sP, o, kk + 4);
-                        fa[i][3] = ldP(sP, o + 8, kk + 4);
-                    }
-#pragma unroll
-                    for(int jn = 0; jn < TN; ++jn)
-                    {
-                        const int n = wn * WN + jn * 8 + g;
-                        fb[jn][0] = ldQ(sQ, n, kk);
-                        fb[jn][1] = ldQ(sQ, n, kk + 4);
+                        advance();
+                        if(kAcross && c + 1 < q.nk)
+                        {
+                            wait_full();
+                            read(0, 0);
+                        }
                     }
 #pragma unroll
                     for(int i = 0; i < TM; ++i)
 #pragma unroll
                         for(int jn = 0; jn < TN; ++jn)
-                            dmma_16x8x8(acc[i][jn], fa[i], fb[jn]);
+                            dmma_16x8x8(acc[ks % SP][i][jn], fa[ks & 1][i], fb[ks & 1][jn]);
                 }
-                const int nxt = kt + Cfg::kStages - 1;
-                if(nxt < nk)
-                {
-                    ok = wait_chunk(nxt);
-                    if(ok)
-                        load_chunk(nxt % Cfg::kStages, nxt);
-                }
-                cp_async_commit();
             }
-            cp_async_wait<0>();
-            __syncthreads();
-            if(!ok)
-                break;
         }
 
-        // ---- 2. T = alpha C_b - acc into shared memory ([row o][col n]) --------------------
+        // ---- 2. T = alpha C_b - sum into shared memory ([row o][col n]), zero outside C_b ---
+        // (rows past the block must not reach the product below, whatever X holds)
 #pragma unroll
         for(int i = 0; i < TM; ++i)
+        {
+            if constexpr(!kEarlyC)
+                read_c(cv[i], i);
 #pragma unroll
             for(int jn = 0; jn < TN; ++jn)
 #pragma unroll
                 for(int e = 0; e < 4; ++e)
                 {
-                    const int o = wm * 32 + i * 16 + g + (e >> 1) * 8;
-                    const int n = wn * WN + jn * 8 + 2 * t + (e & 1);
-                    double    v = 0.0;
-                    if(!zero && o < bs && n < wv)
-                        v = alpha * (double)__ldcg(caddr(r0 + o, c0 + n)) - acc[i][jn][e];
-                    Ts[o * Cfg::kPitchT + n] = v;
+                    const int o = out_o(i, e), col = out_n(jn, e);
+                    double    v = acc[0][i][jn][e];
+#pragma unroll
+                    for(int s = 1; s < SP; ++s)
+                    {
+                        v += acc[s][i][jn][e];
+                        acc[s][i][jn][e] = 0.0;
+                    }
+                    acc[0][i][jn][e] = 0.0;
+                    Ts[o * Cfg::kPitchT + col] = o < q.bs && col < q.wv ? cv[i][jn][e] - v : 0.0;
                 }
-
-        // ---- 3. X_b = inv(M_bb) T: invA chunks through the pipeline, T resident ---------
-        // inv(M_bb)(o, kk) = tM ? invA(kk, o) : invA(o, kk); its triangle: lower when M is
-        // lower (forward), upper otherwise; rows / columns >= bs are zero.
-#pragma unroll
-        for(int i = 0; i < TM; ++i)
-#pragma unroll
-            for(int jn = 0; jn < TN; ++jn)
-#pragma unroll
-                for(int e = 0; e < 4; ++e)
-                    acc[i][jn][e] = 0.0;
-        const int nki = (int)ceil_div(bs, Cfg::kBK);
-        auto load_inv = [&](int stage, int c) {
-            T*        sP = smem + stage * Cfg::kStage;
-            const int k0 = c * Cfg::kBK;
-#pragma unroll
-            for(int i = 0; i < kChainNB * Cfg::kBK / kChainThreads; ++i)
-            {
-                const int e = tid + i * kChainThreads;
-                int       o, kk;
-                if(KCP) { kk = e % Cfg::kBK; o = e / Cfg::kBK; }
-                else    { o = e % kChainNB; kk = e / kChainNB; }
-                const int  kr    = k0 + kk;
-                const bool tri   = forward ? kr <= o : kr >= o;
-                const bool valid = !zero && o < bs && kr < bs && tri;
-                const T*   src   = valid ? (KCP ? inv + kr + (int64_t)o * kChainNB
-                                                : inv + o + (int64_t)kr * kChainNB)
-                                         : inv;
-                T* dst = KCP ? sP + o * Cfg::kPitchP + kk : sP + kk * Cfg::kPitchP + o;
-                chain_cp_async<T>(dst, src, valid);
-            }
-        };
-#pragma unroll 1
-        for(int s = 0; s < Cfg::kStages - 1; ++s)
-        {
-            if(s < nki)
-                load_inv(s, s);
-            cp_async_commit();
+            asm volatile("" ::: "memory"); // the next rows' reads stay behind (registers)
         }
+        asm volatile("barrier.cta.sync 1, %0;" ::"n"(kChainMmaThreads) : "memory");
+
+        // ---- 3. X_b = inv(M_bb) T: chunks of the inverse through the ring, T resident ---------
+        // k steps wholly outside the triangle of this warp's rows are skipped
 #pragma unroll 1
-        for(int kt = 0; kt < nki; ++kt)
+        for(int c = 0; c < q.nki; ++c)
         {
-            cp_async_wait<Cfg::kStages - 2>();
-            __syncthreads();
-            const T* sP = smem + (kt % Cfg::kStages) * Cfg::kStage;
+            const T* sP = ring + st * Cfg::kStage;
+            wait_bar(&full[st], ph);
 #pragma unroll
-            for(int ks = 0; ks < Cfg::kBK / 8; ++ks)
+            for(int ks = 0; ks < BK / 8; ++ks)
             {
-                const int kk = ks * 8 + t;
-                const int kg = kt * Cfg::kBK + kk; // row of T
-                double    fa[TM][4], fb[TN][2];
+                const int kb = c * BK + ks * 8; // row of T
+                if(q.forward ? kb > row0 + Cfg::kWM - 1 : kb + 7 < row0)
+                    continue;
+                double fa[TM][4], fb[TN][2];
+                load_a(fa, sP, ks * 8 + t);
+                // entries outside the triangle, in the k steps that touch the warp's rows
+                if(q.forward ? kb + 7 > row0 : kb < row0 + Cfg::kWM - 1)
 #pragma unroll
-                for(int i = 0; i < TM; ++i)
-                {
-                    const int o = wm * 32 + i * 16 + g;
-                    fa[i][0] = ldP(sP, o, kk);
-                    fa[i][1] = ldP(sP, o + 8, kk);
-                    fa[i][2] = ldP(sP, o, kk + 4);
-                    fa[i][3] = ldP(sP, o + 8, kk + 4);
-                }
+                    for(int i = 0; i < TM; ++i)
+#pragma unroll
+                        for(int e = 0; e < 4; ++e)
+                        {
+                            const int o = out_o(i, 2 * (e & 1)), kr = kb + t + 4 * (e >> 1);
+                            if(q.forward ? kr > o : kr < o)
+                                fa[i][e] = 0.0;
+                        }
 #pragma unroll
                 for(int jn = 0; jn < TN; ++jn)
                 {
-                    const int n = wn * WN + jn * 8 + g;
-                    fb[jn][0] = Ts[kg * Cfg::kPitchT + n];
-                    fb[jn][1] = Ts[(kg + 4) * Cfg::kPitchT + n];
+                    const int nn = col0 + jn * 8 + g;
+                    fb[jn][0] = Ts[(kb + t) * Cfg::kPitchT + nn];
+                    fb[jn][1] = Ts[(kb + t + 4) * Cfg::kPitchT + nn];
                 }
 #pragma unroll
                 for(int i = 0; i < TM; ++i)
 #pragma unroll
                     for(int jn = 0; jn < TN; ++jn)
-                        dmma_16x8x8(acc[i][jn], fa[i], fb[jn]);
+                        dmma_16x8x8(acc[ks % SP][i][jn], fa[i], fb[jn]);
             }
-            const int nxt = kt + Cfg::kStages - 1;
-            if(nxt < nki)
-                load_inv(nxt % Cfg::kStages, nxt);
-            cp_async_commit();
+            advance();
         }
-        cp_async_wait<0>();
 
         // ---- 4. X_b over C_b, then release the item's flag ---------------------------------
+        const bool live = !aborted();
 #pragma unroll
         for(int i = 0; i < TM; ++i)
 #pragma unroll
@@ -507,14 +770,20 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
 #pragma unroll
                 for(int e = 0; e < 4; ++e)
                 {
-                    const int o = wm * 32 + i * 16 + g + (e >> 1) * 8;
-                    const int n = wn * WN + jn * 8 + 2 * t + (e & 1);
-                    if(o < bs && n < wv)
-                        *caddr(r0 + o, c0 + n) = (T)acc[i][jn][e];
+                    const int o = out_o(i, e), col = out_n(jn, e);
+                    double    v = acc[0][i][jn][e];
+#pragma unroll
+                    for(int s = 1; s < SP; ++s)
+                        v += acc[s][i][jn][e];
+                    if(live && o < q.bs && col < q.wv)
+                        *caddr(o, col) = (T)v;
                 }
-        __syncthreads();
+        // all of X_b is written (and T free for the next item) once every MMA warp is here
+        if(mma_sync_stop())
+            break;
         if(tid == 0)
-            chain_st_release(flags + item, 1);
+            chain_st_release((VB ? p.vhdr->flags : p.flags) + q.item, 1);
+        item_done(n);
     }
 }
 
@@ -552,7 +821,7 @@ template <typename T, int W, bool KCP, bool KCQ, bool VB>
 static void launch_chain_cfg(const ChainParams<T>& p, int sms, int64_t max_items, cudaStream_t s,
                              bool cluster2 = false)
 {
-    using Cfg = ChainCfg<T, W, KCP, KCQ, VB>;
+    using Cfg = ChainCfg<T, W, KCP, KCQ>;
     auto kern = trsm_chain_kernel<T, W, KCP, KCQ, VB>;
     cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem);
     int per_sm = 0;
@@ -582,7 +851,7 @@ static void launch_chain_cfg(const ChainParams<T>& p, int sms, int64_t max_items
 }
 
 template <typename T, int W, bool VB>
-static void launch_chain_w(const ChainParams<T>& p, bool kcp, bool kcq, int sms, int64_t max_items,
+void launch_chain_w(const ChainParams<T>& p, bool kcp, bool kcq, int sms, int64_t max_items,
                            cudaStream_t s, bool cluster2 = false)
 {
     if(kcp && kcq)
@@ -594,5 +863,19 @@ static void launch_chain_w(const ChainParams<T>& p, bool kcp, bool kcq, int sms,
     else
         launch_chain_cfg<T, W, false, false, VB>(p, sms, max_items, s, cluster2);
 }
+
+// instantiated in chain_kernels.cu
+extern template void launch_chain_w<double, 8, false>(const ChainParams<double>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<double, 16, false>(const ChainParams<double>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<double, 32, false>(const ChainParams<double>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<double, 64, false>(const ChainParams<double>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<double, 32, true>(const ChainParams<double>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<double, 64, true>(const ChainParams<double>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<float, 8, false>(const ChainParams<float>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<float, 16, false>(const ChainParams<float>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<float, 32, false>(const ChainParams<float>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<float, 64, false>(const ChainParams<float>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<float, 32, true>(const ChainParams<float>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<float, 64, true>(const ChainParams<float>&, bool, bool, int, int64_t, cudaStream_t, bool);
 
 } // namespace rb200

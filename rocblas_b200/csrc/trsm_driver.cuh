@@ -65,6 +65,7 @@ struct TrsmProblem
     int*        err_dev;  // device error word of the bounded waits (or nullptr)
     int         crt_pair_ok = 0; // the residue GEMM may run as CTA pairs on sm_count SMs that
                                  // are whole SM pairs (set beside a kernel placed in pairs)
+    int         chain_w = 0; // strip width of the chain solve (0: chain_width's choice)
     int         k() const { return side_left ? m : n; }
     // op(A) lower?
     int oplower() const { return (!upper) != (trans != 0); }
@@ -352,12 +353,43 @@ static bool use_chain(const TrsmProblem<T>& pr)
     return pr.k() > kInvNB && ncols <= limit;
 }
 
+// Strip width of a uniform chain solve.  Two things bound it: the chain of nb blocks, each of which
+// costs its products (which shrink with the width) and a fixed hand-off, and the rate at which the
+// SMs do the whole work (which falls with the width, because every strip reads all of M from L2:
+// at 8 columns that, not the tensor pipe, is the limit).  The times below are measured per width
+// (one B200, FP64; FP32 systems compute the same): microseconds per block of a chain with one
+// right-hand side (m = 8192), and TFLOP/s at m = n = 8192.  They add up as sqrt(a^2 + b^2), which
+// is within 15% of what was measured from 512 x 256 to 8192 x 8192.
+static int chain_width(int k, int64_t ncols, int systems, int sms)
+{
+    const int forced = tuning().chain_w;
+    if(forced == 8 || forced == 16 || forced == 32 || forced == 64)
+        return forced;
+    constexpr int    kW[]    = {8, 16, 32, 64};
+    constexpr double kStep[] = {5.7, 8.2, 12.6, 24.0};   // us per block
+    constexpr double kRate[] = {13.5, 24.0, 30.4, 30.8}; // TFLOP/s on 148 SMs
+    int              best = 64;
+    double           least = 0.0;
+    for(int i = 0; i < 4; ++i)
+    {
+        const double nb = (double)ceil_div(k, kChainNB), chain = nb * kStep[i];
+        const double flops = (double)k * k * (double)(ceil_div(ncols, kW[i]) * kW[i]) * systems;
+        const double work  = flops / (kRate[i] * 1e6 * sms / 148.0);
+        const double cost  = chain * chain + work * work;
+        if(i == 0 || cost < least)
+        {
+            least = cost;
+            best  = kW[i];
+        }
+    }
+    return best;
+}
+
 template <typename T>
 static ChainShape chain_shape_of(const TrsmProblem<T>& pr)
 {
     const int ncols = pr.side_left ? pr.n : pr.m;
-    const int t     = tuning().chain_w;
-    const int w     = t == 32 || t == 64 ? t : (ncols <= 32 ? 32 : 64);
+    const int w     = pr.chain_w ? pr.chain_w : chain_width(pr.k(), ncols, pr.batch, pr.sm_count);
     return chain_shape(pr.k(), ncols, pr.batch, w);
 }
 
@@ -412,7 +444,9 @@ static void launch_chain_sub(const TrsmProblem<T>& pr, int b0, int b1, int first
     // KCP: M's column index (K) is contiguous in memory when M(r, c) = A(c, r)
     const bool tM  = pr.trans != (pr.side_left ? 0 : 1);
     const bool kcq = pr.side_left != 0;
-    if(w == 16)
+    if(w == 8)
+        launch_chain_w<T, 8, false>(c, tM, kcq, pr.sm_count, cs.items, pr.stream, cluster2);
+    else if(w == 16)
         launch_chain_w<T, 16, false>(c, tM, kcq, pr.sm_count, cs.items, pr.stream, cluster2);
     else if(w == 32)
         launch_chain_w<T, 32, false>(c, tM, kcq, pr.sm_count, cs.items, pr.stream, cluster2);

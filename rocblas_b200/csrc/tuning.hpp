@@ -31,7 +31,7 @@ struct Tuning
     int oz_bk                = 64;   // sliced GEMM K step in int8 (32 or 64)
     int chain_max_cols       = 1 << 30; // FP64 solves (k > 128) with <= this many columns: chain
     int chain_max_cols_f32   = 512;  // the same for FP32 (the chain computes in FP64)
-    int chain_w              = 0;    // chain strip width: 0 auto (32 or 64), 32, 64
+    int chain_w              = 0;    // chain strip width: 8, 16, 32, 64, or 0 (chain_width's choice)
     int mixed_chain_blocks   = 8;    // precision form: chain solves for diagonal blocks of <= this
                                      // many 128-row blocks (< 2: recursion down to the leaves)
     int host_step_blocks     = 4;    // precision form on host buffers: rows per pipelined step,
@@ -39,9 +39,9 @@ struct Tuning
     int sliced_k_chunk       = 16384; // sliced GEMM: K range per set of row / column exponents
                                       // (multiple of 64, at most 16384); shorter ranges keep
                                       // more bits of entries far below their row's maximum
-    int refine_check_sms     = 6;    // refined form: SMs of the FP64 solve of the tested
+    int refine_check_sms     = 4;    // refined form: SMs of the FP64 solve of the tested
                                      // right-hand sides, which runs beside the sliced solve
-    int refine_check_w       = 32;   // refined form: strip width of that solve's chain (16, 32)
+    int refine_check_w       = 8;    // refined form: strip width of that solve's chain (8, 16, 32)
     int refine_check_pairs   = 1;    // refined form: that chain in clusters of two CTAs, so the
                                      // sliced solve beside it may run CTA-pair GEMMs
     int refine_check_flag    = 0;    // refined form: that solve as the memory-bound flag
@@ -92,7 +92,7 @@ static const TuningEntry kTuningEntries[] = {
     {"sliced_k_chunk", &Tuning::sliced_k_chunk, 64, 16384},
     {"refine_check_sms", &Tuning::refine_check_sms, 1, 1024},
     {"refine_check_flag", &Tuning::refine_check_flag, 0, 1},
-    {"refine_check_w", &Tuning::refine_check_w, 16, 32},
+    {"refine_check_w", &Tuning::refine_check_w, 8, 32},
     {"refine_check_pairs", &Tuning::refine_check_pairs, 0, 1},
     {"wait_cycles_log2", &Tuning::wait_cycles_log2, 10, 40},
     {"chain_first_item", &Tuning::chain_first_item, 0, 1 << 30},

@@ -1,0 +1,96 @@
+"""The chain solve (trsm_chain.cuh) at every strip width and at ragged strips, blocks and leading
+dimensions, forward and backward, both element types; a workspace that holds only the widest
+strips' flags is still used; and the inverse-block kernel (trtri_block.cuh) at its tile edges."""
+import ctypes
+import itertools
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import oracle  # noqa: E402
+import rocblas_b200 as rb  # noqa: E402
+from rocblas_b200 import devmem as dm  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def width():
+    L, old = rb.lib(), ctypes.c_int(-1)
+    assert L.rocblas_b200_get_tuning(b"chain_w", ctypes.byref(old)) == 0
+    yield lambda w: L.rocblas_b200_set_tuning(b"chain_w", w)
+    L.rocblas_b200_set_tuning(b"chain_w", old.value)
+
+
+def _solve(h, side, uplo, trans, diag, m, n, A, B):
+    dA, dB = dm.to_device(A), dm.to_device(B)
+    dm.trsm(h, side, uplo, trans, diag, m, n, 1.25, dA, A.shape[0], dB, B.shape[0])
+    torch.cuda.synchronize()
+    return dm.to_host(dB)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("w", [8, 16, 32, 64])
+def test_widths(width, w, dtype):
+    assert width(w) == 0
+    with rb.Handle() as h:
+        for i, (side, uplo, trans, diag) in enumerate(itertools.product("LR", "UL", "NT", "NU")):
+            k, cols = [(129, 1), (257, w), (384, w + 1), (513, 2 * w - 1), (640, 9)][i % 5]
+            m, n = (k, cols) if side == "L" else (cols, k)
+            A, B = oracle.nan_triangle_problem(i, side, uplo, trans, diag, m, n, k + i % 3, m + i % 2, dtype)
+            out = _solve(h, side, uplo, trans, diag, m, n, A, B)
+            X = oracle.trsm(side, uplo, trans, diag, 1.25, A, np.asfortranarray(B[:m]))
+            assert oracle.matrix_norm_1(X, out[:m]) <= oracle.trsm_tolerance(dtype, max(m, n)), (side, uplo, trans, diag)
+            assert np.isnan(out[m:]).all()
+        code = ctypes.c_int(-1)
+        assert rb.lib().rocblas_b200_get_device_error(h.value, ctypes.byref(code)) == 0 and code.value == 0
+
+
+def test_workspace_of_the_widest_strips(width):
+    """A fixed workspace too small for the flags of narrow strips, but large enough for those of
+    the widest: the blocked solve runs, not the degraded one."""
+    k, cols = 1000, 48
+    L = rb.lib()
+
+    def query(h, w):
+        assert width(w) == 0
+        size, a = ctypes.c_size_t(0), ctypes.c_double(1.0)
+        assert L.rocblas_start_device_memory_size_query(h.value) == 0
+        L.rocblas_dtrsm(h.value, rb.side_left, rb.fill_lower, rb.operation_none, rb.diagonal_non_unit, k, cols,
+                        ctypes.cast(ctypes.byref(a), ctypes.c_void_p), None, k, None, k)
+        assert L.rocblas_stop_device_memory_size_query(h.value, ctypes.byref(size)) == 0
+        return size.value
+
+    with rb.Handle() as h:
+        wide = query(h, 64)
+        assert query(h, 8) > wide
+        assert L.rocblas_set_device_memory_size(h.value, wide) == 0
+        A, B = oracle.nan_triangle_problem(5, "L", "L", "N", "N", k, cols, k, k, np.float64)
+        out = _solve(h, "L", "L", "N", "N", k, cols, A, B)  # status success, not perf_degraded
+        X = oracle.trsm("L", "L", "N", "N", 1.25, A, B)
+        assert oracle.matrix_norm_1(X, out) <= oracle.trsm_tolerance(np.float64, k)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 32, 33, 64, 65, 127, 128, 200])
+def test_inverse_blocks(n, dtype):
+    rng = np.random.default_rng(n)
+    with rb.Handle() as h:
+        for uplo, diag in itertools.product("UL", "NU"):
+            A = rng.uniform(-1, 1, (n, n)) / n
+            A = np.tril(A, -1) if uplo == "L" else np.triu(A, 1)
+            T = A + (np.eye(n) if diag == "U" else np.diag(rng.uniform(1, 2, n)))
+            stored = np.where(np.eye(n, dtype=bool) & (diag == "U"), np.nan, T)
+            other = np.triu(np.ones((n, n), bool), 1) if uplo == "L" else np.tril(np.ones((n, n), bool), -1)
+            stored[other] = np.nan
+            dA = dm.to_device(np.asfortranarray(stored, dtype=dtype))
+            dX = dm.empty(n + 1, n, dA.dtype, fill=0.0)
+            dm.trtri(h, uplo, diag, n, dA, n, dX, n + 1)
+            torch.cuda.synchronize()
+            X = dm.to_host(dX)[:n]
+            eps = np.finfo(dtype).eps
+            # the inverse's entries are at most about 1; n terms per product
+            assert np.abs(X - np.linalg.inv(T.astype(dtype).astype(np.float64))).max() <= 4 * n * eps
+            assert (X[other] == 0).all()
