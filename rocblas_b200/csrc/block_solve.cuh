@@ -1,4 +1,5 @@
-// One-CTA triangular solve of a strip of right-hand sides, for small and batched systems.
+// One-CTA triangular solve of a strip of right-hand sides, complex types, for small and batched
+// systems (real types: strip_solve.cuh).
 //
 // Replaces the reference's small and substitution kernels
 // (library/src/blas3/rocblas_trsm_kernels.hpp: rocblas_trsm_small_right_device :1962-2227,
@@ -15,19 +16,17 @@
 // shared memory, and walks the diagonal in 32-row panels:
 //   1. stage the 32 x 32 diagonal tile of M (reciprocal diagonal precomputed, as the
 //      reference does at :3204-3219);
-//   2. forward substitution of the diagonal tile: for real types one warp solves it, one
-//      column per lane held in registers, with the tile's entries broadcast from shared
-//      memory; complex types, whose column would need too many registers, spread the columns
-//      over the warps and broadcast each solved row value with __shfl_sync (the reference
-//      broadcasts through LDS with two __syncthreads per row, :3225-3248);
+//   2. forward substitution of the diagonal tile: the columns spread over the warps, each solved
+//      row value broadcast with __shfl_sync (the reference broadcasts through LDS with two
+//      __syncthreads per row, :3225-3248);
 //   3. rank-32 update of the remaining rows from panels of M streamed through shared
 //      memory in 64-row chunks.
-// k is at most kBlockSolveMaxK; larger systems use the blocked recursive path.
+// k is at most block_solve_max_k; larger systems use the blocked recursive path.
 #pragma once
 #include <type_traits>
 
 #include "common.cuh"
-#include "mma_f64.cuh"
+#include "strip_solve.cuh"
 
 namespace rb200
 {
@@ -36,90 +35,20 @@ constexpr int kBsW       = 32;  // right-hand sides per CTA
 constexpr int kBsPitch   = kBsW + 1;
 constexpr int kBsThreads = 256;
 constexpr int kBsChunk   = 64;  // panel rows per update chunk
-constexpr int kBlockSolveMaxK = 512;
 
-// The largest order one CTA solves: the k x 32 strip of C lives in shared memory, so complex
-// double (16-byte elements) stops at 256 to stay within 227 KB.
+// The largest order one CTA solves.  Complex: the k x 32 strip of C lives in shared memory, so
+// complex double (16-byte elements) stops at 256 to stay within 227 KB.
 template <typename T>
 __host__ __device__ constexpr int block_solve_max_k()
 {
-    return sizeof(T) > 8 ? 256 : kBlockSolveMaxK;
-}
-
-// One system (or a uniform batch of systems).
-template <typename T>
-struct BlockSolveParams
-{
-    int         m, n, k;        // B is m x n; A is k x k
-    int         side_left;
-    int         tM;             // M(i,j) = tM ? A(j,i) : A(i,j)
-    int         rev;            // M upper: rows reversed
-    int         unit;
-    int         conj;           // M's entries are conjugated (complex trans C)
-    BatchPtr<T> A;
-    int64_t     lda;
-    BatchPtr<T> B;
-    int64_t     ldb;
-    Scalar<T>   ualpha;         // the caller's alpha
-    int         first;          // 1: this solve applies ualpha; 0: it applies 1
-    int         batch_base;
-};
-
-// Row pitches (elements) of the strip C and of the streamed panel chunk in shared memory.  FP64
-// runs the update on DMMA, whose fragment reads (lanes (g, t) reading element (g, t) of the
-// chunk and (t, g) of the solved rows) fall on distinct bank pairs of each half-warp with a
-// pitch of 36; FP32 reads the chunk as float4, which a pitch of 36 keeps 16-byte aligned.
-// Other types keep 33, which makes the column reads of the substitution conflict-free.
-template <typename T>
-__host__ __device__ constexpr int bs_cpitch()
-{
-    return std::is_same<T, double>::value ? 36 : kBsPitch;
-}
-template <typename T>
-__host__ __device__ constexpr int bs_ppitch()
-{
-    return std::is_same<T, double>::value || std::is_same<T, float>::value ? 36 : kBsPitch;
+    return is_cplx<T>::value && sizeof(T) > 8 ? 256 : kSsMaxK;
 }
 
 template <typename T>
 __host__ __device__ constexpr size_t block_solve_smem_bytes(int k)
 {
     const int kpad = (int)ceil_div(k, 32) * 32;
-    return sizeof(T) * (size_t)(kpad * bs_cpitch<T>() + 32 * 33 + 32 + kBsChunk * bs_ppitch<T>());
-}
-
-// FP64 update of one chunk on the tensor path: C[0:rows, 0:32] -= P[0:64, 0:32] X[0:32, 0:32]
-// (P: the chunk of M, pitch 36; X: the solved panel rows and C: the rows below, pitch 36; rows
-// >= `rows` do not exist and are not written).  Warp w owns rows 16 (w % 4) .. + 16 and columns
-// 16 (w / 4) .. + 16: two mma.sync m16n8k8 tiles per 8-deep k step, 8 MMAs per warp.
-__device__ __forceinline__ void bs_update_dmma(const double* Ps, const double* Xs, double* Cc,
-                                               int rows, int warp, int lane)
-{
-    constexpr int P = 36;
-    const int     wr = (warp & 3) * 16, wc = (warp >> 2) * 16;
-    const int     g = lane >> 2, t = lane & 3;
-    double        acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-#pragma unroll
-    for(int ks = 0; ks < 32; ks += 8)
-    {
-        const double a[4] = {Ps[(wr + g) * P + ks + t], Ps[(wr + g + 8) * P + ks + t],
-                             Ps[(wr + g) * P + ks + t + 4], Ps[(wr + g + 8) * P + ks + t + 4]};
-#pragma unroll
-        for(int j = 0; j < 2; ++j)
-        {
-            const double b[2] = {Xs[(ks + t) * P + wc + 8 * j + g], Xs[(ks + t + 4) * P + wc + 8 * j + g]};
-            dmma_16x8x8(acc[j], a, b);
-        }
-    }
-#pragma unroll
-    for(int j = 0; j < 2; ++j)
-#pragma unroll
-        for(int e = 0; e < 4; ++e)
-        {
-            const int r = wr + g + (e >> 1) * 8, c = wc + 8 * j + 2 * t + (e & 1);
-            if(r < rows)
-                Cc[r * P + c] -= acc[j][e];
-        }
+    return sizeof(T) * (size_t)(kpad * kBsPitch + 32 * 33 + 32 + kBsChunk * kBsPitch);
 }
 
 // The core: solve M Y = alpha C for one strip.  The caller resolves pointers / sizes.
@@ -128,7 +57,8 @@ __device__ void block_solve_strip(const T* A, int64_t lda, T* B, int64_t ldb, in
                                   int side_left, int tM, int rev, int unit, int conj, T alpha,
                                   int s0, int ncols, unsigned char* smem_raw)
 {
-    constexpr int PC = bs_cpitch<T>(), PP = bs_ppitch<T>();
+    static_assert(is_cplx<T>::value, "real types: strip_solve.cuh");
+    constexpr int PC = kBsPitch, PP = kBsPitch;
     constexpr int NW = kBsThreads / 32; // warps
     T* Cs    = reinterpret_cast<T*>(smem_raw);
     const int kpad = ((k + 31) / 32) * 32;
@@ -274,32 +204,8 @@ __device__ void block_solve_strip(const T* A, int64_t lda, T* B, int64_t ldb, in
             fetch_chunk(p, p + 32);
 
         // ---- 2. substitution of the 32 x 32 diagonal tile ------------------------------------
-        // One warp, one column per lane held in registers: y_j *= 1/M_jj, then
-        // y_i -= M_ij y_j for i > j (the reference's column order); M_ij is a shared-memory
-        // broadcast.  Complex types (64 / 128 registers for the column) broadcast solved rows by
-        // shuffle across all warps instead: warp w owns columns w, w+8, w+16, w+24, lane = row.
-        if constexpr(!is_cplx<T>::value)
-        {
-            if(warp == 0)
-            {
-                T y[32];
-#pragma unroll
-                for(int i = 0; i < 32; ++i)
-                    y[i] = Cs[(p + i) * PC + lane];
-#pragma unroll
-                for(int j = 0; j < 32; ++j)
-                {
-                    y[j] *= rdiag[j];
-#pragma unroll
-                    for(int i = j + 1; i < 32; ++i)
-                        y[i] -= Ds[i * 33 + j] * y[j];
-                }
-#pragma unroll
-                for(int i = 0; i < 32; ++i)
-                    Cs[(p + i) * PC + lane] = y[i];
-            }
-        }
-        else
+        // Solved rows are broadcast by shuffle: warp w owns columns w, w+8, w+16, w+24, lane = row
+        // (a column per lane would need 64 or 128 registers).
         {
             T y[4];
 #pragma unroll
@@ -327,15 +233,6 @@ __device__ void block_solve_strip(const T* A, int64_t lda, T* B, int64_t ldb, in
         __syncthreads();
 
         // ---- 3. update rows p+32 .. k-1 (chunks prefetched one step ahead) ----------------
-        // FP32 keeps this thread's column of the solved panel in registers for all chunks
-        float xr[std::is_same<T, float>::value ? 32 : 1];
-        if constexpr(std::is_same<T, float>::value)
-        {
-            if(p + 32 < k)
-#pragma unroll
-                for(int t = 0; t < 32; ++t)
-                    xr[t] = Cs[(p + t) * PC + lane];
-        }
         for(int i0 = p + 32; i0 < k; i0 += kBsChunk)
         {
             store_chunk();
@@ -344,28 +241,6 @@ __device__ void block_solve_strip(const T* A, int64_t lda, T* B, int64_t ldb, in
                 fetch_chunk(p, i0 + kBsChunk);
             else
                 fetch_diag(p + 32); // p + 32 < k here
-            if constexpr(std::is_same<T, double>::value)
-            {
-                bs_update_dmma(Ps, Cs + (size_t)p * PC, Cs + (size_t)i0 * PC, kpad - i0, warp, lane);
-            }
-            else if constexpr(std::is_same<T, float>::value)
-            {
-#pragma unroll
-                for(int q = 0; q < kBsChunk / NW; ++q)
-                {
-                    const int r   = warp + NW * q;
-                    float     acc = 0.0f;
-#pragma unroll
-                    for(int t = 0; t < 32; t += 4)
-                    {
-                        const float4 m4 = *reinterpret_cast<const float4*>(&Ps[r * PP + t]);
-                        acc += m4.x * xr[t] + m4.y * xr[t + 1] + m4.z * xr[t + 2] + m4.w * xr[t + 3];
-                    }
-                    if(i0 + r < kpad)
-                        Cs[(i0 + r) * PC + lane] -= acc;
-                }
-            }
-            else
             {
                 const int col = lane;
 #pragma unroll

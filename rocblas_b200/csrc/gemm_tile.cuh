@@ -18,6 +18,7 @@
 // them.  The same holds for side right with P == C and N <= BN.  b must be 0 then.
 #pragma once
 #include "common.cuh"
+#include "mma_f64.cuh"
 
 namespace rb200
 {
@@ -111,13 +112,6 @@ struct TileStage
         }
     }
 };
-
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
 
 template <typename T>
 struct GemmAcc;

@@ -16,6 +16,15 @@ __device__ __forceinline__ void dmma_16x8x8(double (&d)[4], const double (&a)[4]
                  : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
+// mma.sync m8n8k4 .f64 (256 FMAs).  Fragments: A (8x4): a (g, t); B (4x8): b (t, g); C (8x8):
+// c0 (g, 2t), c1 (g, 2t+1).
+__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
 // mma.sync m16n8k16 .f64: the k8 fragments of two consecutive k8 steps side by side,
 // a_{2q+r} = A(g + 8r, t + 4q), b_q = B(t + 4q, g) for q = 0..3, r = 0..1.
 __device__ __forceinline__ void dmma_16x8x16(double (&d)[4], const double (&a)[8], const double (&b)[4])

@@ -1185,15 +1185,19 @@ void launch_vb_queue(rocblas_handle h, const VbParams<T>& p, int kmax)
         count_launch();
         return;
     }
-    const size_t smem = block_solve_smem_bytes<T>(std::max(kmax, 1));
-    cudaFuncSetAttribute((const void*)vb_persistent_kernel<T>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vb_persistent_kernel<T>, kBsThreads, smem);
-    per_sm = std::max(per_sm, 1);
-    TimedLaunch tl(KernelClass::strip, h->stream, 0.0);
-    vb_persistent_kernel<T><<<h->sm_count * per_sm, kBsThreads, smem, h->stream>>>(p);
-    count_launch();
+    auto launch = [&](auto kern, size_t smem) {
+        cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSsThreads, smem);
+        per_sm = std::max(per_sm, 1);
+        TimedLaunch tl(KernelClass::strip, h->stream, 0.0);
+        kern<<<h->sm_count * per_sm, kSsThreads, smem, h->stream>>>(p);
+        count_launch();
+    };
+    if(kmax <= 64)
+        launch(vb_persistent_kernel<T, 8, 2, 5>, SsCfg<T, 8, 2>::kSmem);
+    else
+        launch(vb_persistent_kernel<T, 16, 2, 3>, SsCfg<T, 16, 2>::kSmem);
 }
 
 template <typename T>
@@ -1204,7 +1208,7 @@ rocblas_status trsm_vbatched_impl(rocblas_handle h, const T* alpha,
     DeviceScope device_scope; // the caller's current device is restored on return
     if(!h)
         return rocblas_status_invalid_handle;
-    if(count < 0 || max_k < 0 || max_k > kBlockSolveMaxK)
+    if(count < 0 || max_k < 0 || max_k > kSsMaxK)
         return rocblas_status_invalid_size;
     const size_t ws_bytes
         = sizeof(VbClassState) + sizeof(int) * (size_t)kVbClasses * ((size_t)count + 1);
@@ -1456,7 +1460,7 @@ rocblas_status trsm_vbatched_noalloc_impl(rocblas_handle h, const double* alpha,
     DeviceScope device_scope; // the caller's current device is restored on return
     if(!h)
         return rocblas_status_invalid_handle;
-    if(count < 0 || max_k < 0 || max_k > kBlockSolveMaxK)
+    if(count < 0 || max_k < 0 || max_k > kSsMaxK)
         return rocblas_status_invalid_size;
     if(count > kVbNoAllocMaxCount)
     {

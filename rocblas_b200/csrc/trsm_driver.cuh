@@ -30,6 +30,7 @@
 #include "gemm_dmma.cuh"
 #include "gemm_tile.cuh"
 #include "handle.hpp"
+#include "strip_solve.cuh"
 #include "trsm_chain.cuh"
 #include "trtri_block.cuh"
 #include "tuning.hpp"
@@ -159,15 +160,22 @@ static void launch_block_solve(const TrsmProblem<T>& pr, int m, int n, BatchPtr<
     p.first  = first;
     const int    ncols   = pr.side_left ? n : m;
     const int    nstrips = (int)ceil_div(ncols, kBsW);
-    const size_t smem    = block_solve_smem_bytes<T>(p.k);
-    ensure_smem_attr<T>((const void*)block_solve_kernel<T>, block_solve_smem_bytes<T>(block_solve_max_k<T>()));
-    for(int b0 = 0; b0 < pr.batch; b0 += kMaxGridYZ)
-    {
-        p.batch_base = b0;
-        dim3 grid((unsigned)nstrips, (unsigned)std::min(kMaxGridYZ, pr.batch - b0));
-        block_solve_kernel<T><<<grid, kBsThreads, smem, pr.stream>>>(p);
-        count_launch();
-    }
+    auto launch = [&](auto kern, int threads, size_t smem) {
+        ensure_smem_attr<T>((const void*)kern, smem);
+        for(int b0 = 0; b0 < pr.batch; b0 += kMaxGridYZ)
+        {
+            p.batch_base = b0;
+            dim3 grid((unsigned)nstrips, (unsigned)std::min(kMaxGridYZ, pr.batch - b0));
+            kern<<<grid, threads, smem, pr.stream>>>(p);
+            count_launch();
+        }
+    };
+    if constexpr(is_cplx<T>::value)
+        launch(block_solve_kernel<T>, kBsThreads, block_solve_smem_bytes<T>(p.k));
+    else if(p.k <= 64)
+        launch(strip_solve_kernel<T, 8, 2, 5>, kSsThreads, SsCfg<T, 8, 2>::kSmem);
+    else
+        launch(strip_solve_kernel<T, 16, 2, 3>, kSsThreads, SsCfg<T, 16, 2>::kSmem);
 }
 
 // ---- recursive blocked solve --------------------------------------------------------------

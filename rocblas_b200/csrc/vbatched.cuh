@@ -17,7 +17,7 @@
 //      instead (vb_warp_kernel).  There is no inter-CTA waiting, so no wait can hang.
 // All launches are stream-ordered and capturable in a CUDA graph.
 #pragma once
-#include "block_solve.cuh"
+#include "strip_solve.cuh"
 
 namespace rb200
 {
@@ -44,7 +44,7 @@ __host__ __device__ constexpr int vb_class_kmax(int c)
 {
     return 32 << c;
 }
-static_assert(vb_class_kmax(kVbClasses - 1) == kBlockSolveMaxK, "classes cover the strip solver");
+static_assert(vb_class_kmax(kVbClasses - 1) == kSsMaxK, "classes cover the strip solver");
 
 __device__ __forceinline__ int vb_class(int k)
 {
@@ -87,7 +87,7 @@ __device__ __forceinline__ int vb_items(const VbProblem& p)
     const int k     = p.side == kLeft ? p.m : p.n;
     if(k == 0 || ncols == 0)
         return 0;
-    return (ncols + kBsW - 1) / kBsW;
+    return (ncols + kSsW - 1) / kSsW;
 }
 
 // offsets[i] = number of work items of problems 0..i-1; offsets[count] = total.
@@ -211,13 +211,13 @@ struct VbParams
     Scalar<T>        alpha;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kBsThreads, 2) vb_persistent_kernel(VbParams<T> p)
+template <typename T, int RT, int NS, int CTAS>
+__global__ void __launch_bounds__(kSsThreads, CTAS) vb_persistent_kernel(VbParams<T> p)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_item;
-    const int total = p.offsets[p.count];
-    const T   alpha = p.alpha.get();
+    const int    total = p.offsets[p.count];
+    const double alpha = (double)p.alpha.get();
     for(;;)
     {
         if(threadIdx.x == 0)
@@ -246,9 +246,8 @@ __global__ void __launch_bounds__(kBsThreads, 2) vb_persistent_kernel(VbParams<T
         const int tM    = trans != (left ? 0 : 1);
         const int oplow = (q.uplo == kLower) != (trans != 0);
         const int mlow  = left ? oplow : !oplow;
-        block_solve_strip<T>(reinterpret_cast<const T*>(q.A), q.lda, reinterpret_cast<T*>(q.B),
-                             q.ldb, k, left, tM, !mlow, q.diag == kUnit, 0, alpha, strip * kBsW,
-                             ncols, smem_raw);
+        strip_solve<T, RT, NS>(reinterpret_cast<const T*>(q.A), q.lda, reinterpret_cast<T*>(q.B), q.ldb, k, left, tM,
+                               !mlow, q.diag == kUnit, alpha, strip * kSsW, ncols, smem_raw);
         __syncthreads();
     }
 }
@@ -274,7 +273,7 @@ __device__ void warp_strip_solve(const T* A, int64_t lda, T* B, int64_t ldb, int
                                  int tM, int rev, int unit, T alpha, int s0, int ncols, T* Ws, T* rd)
 {
     const int lane = threadIdx.x & 31;
-    const int W    = min(kBsW, ncols - s0);
+    const int W    = min(kSsW, ncols - s0);
     T* const      B0  = B + (side_left ? (int64_t)s0 * ldb : (int64_t)s0);
     const int64_t bdr = side_left ? 1 : ldb, bdc = side_left ? ldb : 1;
     // C'(i, col): row i of the reversed orientation (rev: C row k-1-i)
@@ -389,7 +388,7 @@ __global__ void __launch_bounds__(32 * kVbWarpsPerCta) vb_warp_kernel(VbParams<T
         const int       oplow = (q.uplo == kLower) != (trans != 0);
         const int       mlow  = left ? oplow : !oplow;
         warp_strip_solve<T>(reinterpret_cast<const T*>(q.A), q.lda, reinterpret_cast<T*>(q.B), q.ldb,
-                            k, left, tM, !mlow, q.diag == kUnit, alpha, strip * kBsW, ncols, Ws, rd);
+                            k, left, tM, !mlow, q.diag == kUnit, alpha, strip * kSsW, ncols, Ws, rd);
     }
 }
 

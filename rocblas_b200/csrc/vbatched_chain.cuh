@@ -25,7 +25,7 @@ constexpr int kChainVbMaxNB   = 256; // chain systems up to k = 32768
 constexpr int kChainVbCombos  = 8;   // (tM, side) x strip width
 constexpr int kChainVbW       = 32;  // the narrow strip width (the flag bound assumes it)
 constexpr int kChainVbWideW   = 64;  // the strip width of systems with more than 32 columns
-constexpr int kChainVbMinK    = kBlockSolveMaxK; // k above this goes to the chain
+constexpr int kChainVbMinK    = kSsMaxK; // k above this goes to the chain
 
 __host__ __device__ constexpr int chain_vb_width(int combo)
 {
