@@ -278,6 +278,11 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
             // a workspace too small for the flags of narrow strips may hold those of the widest
             pr.chain_w = 64;
             ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
+            if(!ws && std::is_same<T, float>::value)
+            {
+                pr.chain_w = -1; // the recursive solve needs no flags
+                ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
+            }
         }
         if(!ws && !have_invA)
         {

@@ -591,7 +591,6 @@ struct MixedRecursive : Recursive<double>
     void* slice_ws;
     int*  err_dev;
     void* chain_ws = nullptr; // flags of the chain sub-solves (nullptr: recursion to the leaves)
-    int   chain_w  = 64;      // and their strip width
     bool  ok = true;
     // optional hooks around every diagonal-block solve of blocks [b0, b1) (a chain sub-solve or
     // a leaf): the host-buffer path waits for A's data before it and copies the finished rows

@@ -66,7 +66,7 @@ struct TrsmProblem
     int*        err_dev;  // device error word of the bounded waits (or nullptr)
     int         crt_pair_ok = 0; // the residue GEMM may run as CTA pairs on sm_count SMs that
                                  // are whole SM pairs (set beside a kernel placed in pairs)
-    int         chain_w = 0; // strip width of the chain solve (0: chain_width's choice)
+    int         chain_w = 0; // strip width of the chain solve (0: chain_width's choice; < 0: no chain)
     int         k() const { return side_left ? m : n; }
     // op(A) lower?
     int oplower() const { return (!upper) != (trans != 0); }
@@ -187,6 +187,10 @@ static bool sliced_trsm_update(const TrsmProblem<T>& q, int c_lo, int c_hi, int 
 static size_t sliced_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int S);
 
 template <typename T>
+static void launch_chain_sub(const TrsmProblem<T>& pr, int b0, int b1, int first, int w, void* ws,
+                             bool cluster2 = false);
+
+template <typename T>
 struct Recursive
 {
     const TrsmProblem<T>& pr;
@@ -194,6 +198,10 @@ struct Recursive
     // FP32: workspace of the trailing updates on the int8 slice engine (nullptr: FFMA tiles)
     void*                 slice_ws = nullptr;
     int                   slice_S  = 0;
+    // diagonal blocks of at most this many 128-row blocks: one chain launch each, its flags in
+    // slice_ws (0: recursion to the leaves)
+    int                   chain_blocks = 0;
+    int                   chain_w      = 64;
 
     int row_of(int b) const { return std::min(b * kInvNB, k); }
 
@@ -290,6 +298,14 @@ struct Recursive
             leaf(b0, first);
             return;
         }
+        if constexpr(!is_cplx<T>::value)
+        {
+            if(b1 - b0 <= chain_blocks)
+            {
+                launch_chain_sub<T>(pr, b0, b1, first, chain_w, slice_ws);
+                return;
+            }
+        }
         const int bm = (b0 + b1) / 2;
         const int r0 = row_of(b0), rm = row_of(bm), r1 = row_of(b1);
         // blocks are solved in increasing order when op(A) is lower (side L) or upper (side R)
@@ -348,17 +364,36 @@ static Algo choose_algo(const TrsmProblem<T>& pr)
                                                                          : Algo::recursive;
 }
 
-// The recursive solve with few right-hand sides runs as one chain launch (trsm_chain.cuh)
-// when invA is available: FP64, more than one 128-row block, at most chain_max_cols columns.
+// The FP32 solve's trailing updates run on the int8 slice engine (strsm_slices > 0, one system,
+// more right-hand sides than chain_max_cols_f32, an update with an inner dimension of
+// strsm_sliced_min_k or more): the larger half at the top node, else 0.
+template <typename T>
+static int64_t strsm_sliced_half(const TrsmProblem<T>& pr)
+{
+    if constexpr(!std::is_same<T, float>::value)
+        return 0;
+    const Tuning& t     = tuning();
+    const int64_t ncols = pr.side_left ? pr.n : pr.m;
+    if(t.strsm_slices <= 0 || pr.batch != 1 || ncols <= t.chain_max_cols_f32)
+        return 0;
+    const int64_t k   = pr.k();
+    const int64_t rm  = std::min<int64_t>(ceil_div(k, kInvNB) / 2 * kInvNB, k);
+    const int64_t big = std::max(rm, k - rm);
+    return big < t.strsm_sliced_min_k ? 0 : big;
+}
+
+// A solve of more than one 128-row block runs as one chain launch (trsm_chain.cuh) when invA is
+// available: FP64 with at most chain_max_cols right-hand sides, FP32 unless its updates are worth
+// the slice engine (or strsm_slices 0 asks for the FFMA recursion).
 template <typename T>
 static bool use_chain(const TrsmProblem<T>& pr)
 {
-    if(is_cplx<T>::value || choose_algo(pr) != Algo::recursive)
+    if(is_cplx<T>::value || choose_algo(pr) != Algo::recursive || pr.chain_w < 0 || pr.k() <= kInvNB)
         return false;
     const int64_t ncols = pr.side_left ? pr.n : pr.m;
-    const int64_t limit = std::is_same<T, double>::value ? tuning().chain_max_cols
-                                                         : tuning().chain_max_cols_f32;
-    return pr.k() > kInvNB && ncols <= limit;
+    if(std::is_same<T, float>::value)
+        return ncols <= tuning().chain_max_cols_f32 || (tuning().strsm_slices > 0 && strsm_sliced_half(pr) == 0);
+    return ncols <= tuning().chain_max_cols;
 }
 
 // Strip width of a uniform chain solve.  Two things bound it: the chain of nb blocks, each of which
@@ -397,7 +432,7 @@ template <typename T>
 static ChainShape chain_shape_of(const TrsmProblem<T>& pr)
 {
     const int ncols = pr.side_left ? pr.n : pr.m;
-    const int w     = pr.chain_w ? pr.chain_w : chain_width(pr.k(), ncols, pr.batch, pr.sm_count);
+    const int w     = pr.chain_w > 0 ? pr.chain_w : chain_width(pr.k(), ncols, pr.batch, pr.sm_count);
     return chain_shape(pr.k(), ncols, pr.batch, w);
 }
 
@@ -408,11 +443,11 @@ __global__ void chain_set_counter_kernel(int* counter, int v)
 
 // Chain solve of the diagonal blocks [b0, b1) of pr (all of it: 0, nblk) with invA available:
 // `first` as in Recursive::solve; `ws` holds chain_workspace_bytes of the sub-problem.
-template <typename T>
 // cluster2: launch the CTAs as clusters of two (placement only: each pair takes both SMs of an SM
 // pair, so that a CTA-pair kernel beside it finds the other SMs in whole pairs)
+template <typename T>
 static void launch_chain_sub(const TrsmProblem<T>& pr, int b0, int b1, int first, int w, void* ws,
-                             bool cluster2 = false)
+                             bool cluster2)
 {
     const int        r0    = b0 * kInvNB;
     const int        kk    = std::min(b1 * kInvNB, pr.k()) - r0;
@@ -474,27 +509,17 @@ static size_t trsm_invA_bytes(const TrsmProblem<T>& pr, bool have_supplied_invA)
     return (size_t)kInvNB * (size_t)pr.k() * sizeof(T) * (size_t)pr.batch;
 }
 
-// The FP32 recursive solve's slice workspace: the largest trailing update (the top node's)
-// when its updates run on the int8 slice engine (strsm_slices > 0, one system, no chain).
+// The FP32 recursive solve's slice workspace: the largest trailing update (the top node's) when
+// its updates run on the int8 slice engine.  The chain sub-solves between the updates keep their
+// flags in the same place.
 template <typename T>
 static size_t strsm_slice_bytes(const TrsmProblem<T>& pr)
 {
-    if constexpr(!std::is_same<T, float>::value)
+    const int64_t big = choose_algo(pr) == Algo::recursive ? strsm_sliced_half(pr) : 0;
+    if(!big)
         return 0;
-    else
-    {
-        const Tuning& t = tuning();
-        if(t.strsm_slices <= 0 || pr.batch != 1 || choose_algo(pr) != Algo::recursive || use_chain(pr))
-            return 0;
-        const int64_t k    = pr.k();
-        const int64_t nblk = ceil_div(k, kInvNB);
-        const int64_t rm   = std::min<int64_t>(nblk / 2 * kInvNB, k);
-        const int64_t big  = std::max(rm, k - rm);
-        if(big < t.strsm_sliced_min_k)
-            return 0;
-        return pr.side_left ? sliced_gemm_workspace_bytes(big, pr.n, big, t.strsm_slices)
-                            : sliced_gemm_workspace_bytes(pr.m, big, big, t.strsm_slices);
-    }
+    const int S = tuning().strsm_slices;
+    return pr.side_left ? sliced_gemm_workspace_bytes(big, pr.n, big, S) : sliced_gemm_workspace_bytes(pr.m, big, big, S);
 }
 
 template <typename T>
@@ -551,6 +576,14 @@ static void trsm_run(TrsmProblem<T> pr, void* ws, bool supplied_invA)
     {
         rec.slice_ws = reinterpret_cast<char*>(ws) + (trsm_invA_bytes(pr, supplied_invA) + 255) / 256 * 256;
         rec.slice_S  = tuning().strsm_slices;
+        // nodes whose update would be too short for the slice engine are chain solves (8192 x 8192:
+        // 2.6 ms where the FFMA updates and leaves took 7.8)
+        const int     nb    = (int)ceil_div(tuning().strsm_sliced_min_k, kInvNB) * 2 - 1;
+        const int64_t ncols = pr.side_left ? pr.n : pr.m;
+        rec.chain_w         = chain_width(nb * kInvNB, ncols, 1, pr.sm_count);
+        if(pr.invA.valid()
+           && chain_workspace_bytes(chain_shape(nb * kInvNB, (int)ncols, 1, rec.chain_w)) <= strsm_slice_bytes(pr))
+            rec.chain_blocks = nb;
     }
     rec.solve(0, rec.nblk, 1);
 }

@@ -30,7 +30,8 @@ struct Tuning
     int oz_bn                = 64;   // sliced GEMM output tile width (64: one pass; 128)
     int oz_bk                = 64;   // sliced GEMM K step in int8 (32 or 64)
     int chain_max_cols       = 1 << 30; // FP64 solves (k > 128) with <= this many columns: chain
-    int chain_max_cols_f32   = 512;  // the same for FP32 (the chain computes in FP64)
+    int chain_max_cols_f32   = 512;  // FP32 solves with more columns: updates on the slice engine
+                                     // where they are deep enough (strsm_sliced_min_k), else chain
     int chain_w              = 0;    // chain strip width: 8, 16, 32, 64, or 0 (chain_width's choice)
     int mixed_chain_blocks   = 8;    // precision form: chain solves for diagonal blocks of <= this
                                      // many 128-row blocks (< 2: recursion down to the leaves)

@@ -94,3 +94,17 @@ def test_inverse_blocks(n, dtype):
             # the inverse's entries are at most about 1; n terms per product
             assert np.abs(X - np.linalg.inv(T.astype(dtype).astype(np.float64))).max() <= 4 * n * eps
             assert (X[other] == 0).all()
+
+
+@pytest.mark.parametrize("k,cols,fixed", [(600, 700, False), (600, 700, True), (1900, 600, False), (2304, 520, False),
+                                          (2400, 530, False)])
+def test_fp32_with_many_columns(k, cols, fixed):
+    """FP32 with more right-hand sides than chain_max_cols_f32: on the chain, or sliced updates
+    between chain sub-solves; in a workspace of the inverse blocks alone, the recursive solve."""
+    A, B = oracle.nan_triangle_problem(k, "L", "L", "N", "N", k, cols, k, k, np.float32)
+    with rb.Handle() as h:
+        if fixed:
+            assert rb.lib().rocblas_set_device_memory_size(h.value, 128 * k * 4) == 0
+        out = _solve(h, "L", "L", "N", "N", k, cols, A, B)  # status success
+    X = oracle.trsm("L", "L", "N", "N", 1.25, A, B)
+    assert oracle.matrix_norm_1(X, out) <= oracle.trsm_tolerance(np.float32, k)
