@@ -21,6 +21,7 @@
 #include "refine.cuh"
 #include "sliced_driver.cuh"
 #include "trsv_flag.cuh"
+#include "trsv_stream.cuh"
 #include "trsm_driver.cuh"
 #include "server.cuh"
 #include "vbatched.cuh"
@@ -549,6 +550,14 @@ void launch_trsv_flag(const TrsvParams<T>& p, int nblk, int sms, cudaStream_t s)
     launch_trsv_flag_nr<T, NB, 1>(p, nblk, sms, s);
 }
 
+template <typename T, bool TR>
+void launch_trsv_stream(const TrsvParams<T>& p, T* xch, int nblk, int sms, cudaStream_t s)
+{
+    constexpr size_t smem = trsv_stream_smem_bytes();
+    cudaFuncSetAttribute((const void*)trsv_stream_kernel<T, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    trsv_stream_kernel<T, TR><<<std::min(nblk, sms), kTsThreads, smem, s>>>(p, xch);
+}
+
 template <typename T>
 rocblas_status trsv_impl(rocblas_handle h, rocblas_fill uplo, rocblas_operation trans,
                          rocblas_diagonal diag, int n, const void* Aptr, BatchPtr<T> A, int64_t lda,
@@ -565,9 +574,12 @@ rocblas_status trsv_impl(rocblas_handle h, rocblas_fill uplo, rocblas_operation 
     {
         if(batch == 1 && incx > 0 && n >= tuning().trsv_flag_min_n)
         {
-            const int    NB    = tuning().trsv_flag_nb == 128 ? 128 : 64;
-            const int    nblk  = (int)ceil_div(n, NB);
-            const size_t bytes = (size_t)nblk * sizeof(int);
+            // blocks of 128 stream with the exchange buffer; the flag solve where the workspace holds
+            // only its flags, or blocks of 64 are asked for
+            const int    NB     = tuning().trsv_flag_nb == 128 ? 128 : 64;
+            const int    nblk   = (int)ceil_div(n, NB);
+            bool         stream = NB == 128;
+            size_t       bytes  = stream ? trsv_stream_workspace_bytes<T>(n) : (size_t)nblk * sizeof(int);
             if(h->size_query)
                 return h->set_optimal_size(bytes);
             rocblas_status st;
@@ -575,6 +587,12 @@ rocblas_status trsv_impl(rocblas_handle h, rocblas_fill uplo, rocblas_operation 
                 return st;
             int*  err = ensure_err(h);
             void* ws  = h->borrow(bytes);
+            if(stream && (!ws || reinterpret_cast<uintptr_t>(ws) % 16)) // the pairs are 16-byte accesses
+            {
+                stream = false;
+                bytes  = (size_t)nblk * sizeof(int);
+                ws     = h->borrow(bytes);
+            }
             if(err && ws)
             {
                 cudaMemsetAsync(ws, 0, bytes, h->stream);
@@ -593,7 +611,11 @@ rocblas_status trsv_impl(rocblas_handle h, rocblas_fill uplo, rocblas_operation 
                 p.flags = reinterpret_cast<int*>(ws);
                 p.error = err;
                 p.wait_cycles = 1ll << tuning().wait_cycles_log2;
-                if(NB == 128)
+                if(stream && p.trans)
+                    launch_trsv_stream<T, true>(p, reinterpret_cast<T*>(ws), nblk, h->sm_count, h->stream);
+                else if(stream)
+                    launch_trsv_stream<T, false>(p, reinterpret_cast<T*>(ws), nblk, h->sm_count, h->stream);
+                else if(NB == 128)
                     launch_trsv_flag<T, 128>(p, nblk, h->sm_count, h->stream);
                 else
                     launch_trsv_flag<T, 64>(p, nblk, h->sm_count, h->stream);

@@ -83,6 +83,78 @@ __device__ __forceinline__ void trtri_mma(double (&acc)[NT][4], const double* P,
     }
 }
 
+// The inverse of the lower triangular 128 x 128 block at X (column-major, pitch kTrtriLd, zero above
+// the diagonal), in place, by 256 threads between two CTA barriers (the caller's before it, the
+// last of its own after it).  Tm: 64 columns of kTrtriLdT doubles.
+__device__ __forceinline__ void trtri_invert(double* X, double* Tm, bool zero_is_one)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    // ---- 16 x 16 diagonal tiles: warp w inverts tile w, lane = column ----------------------------
+    {
+        constexpr int S = 16;
+        double* const D = X + warp * S * (kTrtriLd + 1);
+        double        d = lane < S ? D[lane * (kTrtriLd + 1)] : 1.0;
+        if(zero_is_one && d == 0.0)
+            d = 1.0;
+        const double rd = 1.0 / d;
+        double       x[S];
+#pragma unroll
+        for(int i = 0; i < S; ++i)
+            x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+        for(int c = 0; c < S; ++c)
+        {
+            x[c] *= __shfl_sync(0xffffffffu, rd, c);
+#pragma unroll
+            for(int i = c + 1; i < S; ++i)
+                x[i] -= D[c * kTrtriLd + i] * x[c];
+        }
+        __syncwarp();
+        if(lane < S)
+#pragma unroll
+            for(int i = 0; i < S; ++i)
+                D[lane * kTrtriLd + i] = x[i];
+    }
+    __syncthreads();
+
+    // ---- 16 -> 32 -> 64 -> 128 ----------------------------------------------------------------
+    // Of a doubling from S, the warp takes NT tiles of 16 x 8 at row rb, column cb of pair pr.
+    auto doubling = [&](auto s_const, auto nt_const, int pr, int rb, int cb) {
+        constexpr int S = decltype(s_const)::value, NT = decltype(nt_const)::value;
+        double* const X11 = X + pr * 2 * S * (kTrtriLd + 1);
+        double* const L21 = X11 + S;
+        double* const X22 = X11 + S * (kTrtriLd + 1);
+        double* const Tp  = Tm + pr * S * kTrtriLdT; // its S columns of the temporary
+        double        acc[NT][4] = {};
+        // Tp = L21 X11: X11's column c is zero above row c
+        trtri_mma<NT>(acc, L21 + rb, kTrtriLd, X11 + cb * kTrtriLd, kTrtriLd, cb, S, g, t);
+#pragma unroll
+        for(int n = 0; n < NT; ++n)
+#pragma unroll
+            for(int e = 0; e < 4; ++e)
+            {
+                Tp[(cb + 8 * n + 2 * t + (e & 1)) * kTrtriLdT + rb + g + (e >> 1) * 8] = acc[n][e];
+                acc[n][e] = 0.0;
+            }
+        __syncthreads();
+        // X21 = -X22 Tp, over L21: X22's row r ends at column r
+        trtri_mma<NT>(acc, X22 + rb, kTrtriLd, Tp + cb * kTrtriLdT, kTrtriLdT, 0, rb + 16, g, t);
+#pragma unroll
+        for(int n = 0; n < NT; ++n)
+#pragma unroll
+            for(int e = 0; e < 4; ++e)
+                L21[(cb + 8 * n + 2 * t + (e & 1)) * kTrtriLd + rb + g + (e >> 1) * 8] = -acc[n][e];
+        __syncthreads();
+    };
+    doubling(std::integral_constant<int, 16>{}, std::integral_constant<int, 1>{}, warp >> 1, 0, (warp & 1) * 8);
+    doubling(std::integral_constant<int, 32>{}, std::integral_constant<int, 2>{}, warp >> 2, (warp & 1) * 16,
+             (warp & 2) * 8);
+    // warps w and w + 4 share a scheduler: opposite row blocks give it even work in both products
+    doubling(std::integral_constant<int, 64>{}, std::integral_constant<int, 4>{}, 0,
+             (warp < 4 ? warp : 7 - warp) * 16, (warp >> 2) * 32);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<T> p)
 {
@@ -91,7 +163,6 @@ __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<
     double* Tm = X + kTrtriNB * kTrtriLd;
 
     const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int     g = lane >> 2, t = lane & 3;
     const int     blk   = blockIdx.x;
     const int     batch = p.batch_base + blockIdx.y;
     const int     k     = p.vk ? p.vk[batch] : p.k;
@@ -150,69 +221,8 @@ __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<
     }
     __syncthreads();
 
-    // ---- 16 x 16 diagonal tiles: warp w inverts tile w, lane = column ----------------------------
-    {
-        constexpr int S = 16;
-        double* const D = X + warp * S * (kTrtriLd + 1);
-        double        d = lane < S ? D[lane * (kTrtriLd + 1)] : 1.0;
-        // unit diagonal and padding (staged as 0), and a zero diagonal entry, read as 1
-        d = d == 0.0 ? 1.0 : d;
-        const double rd = 1.0 / d;
-        double       x[S];
-#pragma unroll
-        for(int i = 0; i < S; ++i)
-            x[i] = i == lane ? 1.0 : 0.0;
-#pragma unroll
-        for(int c = 0; c < S; ++c)
-        {
-            x[c] *= __shfl_sync(0xffffffffu, rd, c);
-#pragma unroll
-            for(int i = c + 1; i < S; ++i)
-                x[i] -= D[c * kTrtriLd + i] * x[c];
-        }
-        __syncwarp();
-        if(lane < S)
-#pragma unroll
-            for(int i = 0; i < S; ++i)
-                D[lane * kTrtriLd + i] = x[i];
-    }
-    __syncthreads();
-
-    // ---- 16 -> 32 -> 64 -> 128 ----------------------------------------------------------------
-    // Of a doubling from S, the warp takes NT tiles of 16 x 8 at row rb, column cb of pair pr.
-    auto doubling = [&](auto s_const, auto nt_const, int pr, int rb, int cb) {
-        constexpr int S = decltype(s_const)::value, NT = decltype(nt_const)::value;
-        double* const X11 = X + pr * 2 * S * (kTrtriLd + 1);
-        double* const L21 = X11 + S;
-        double* const X22 = X11 + S * (kTrtriLd + 1);
-        double* const Tp  = Tm + pr * S * kTrtriLdT; // its S columns of the temporary
-        double        acc[NT][4] = {};
-        // Tp = L21 X11: X11's column c is zero above row c
-        trtri_mma<NT>(acc, L21 + rb, kTrtriLd, X11 + cb * kTrtriLd, kTrtriLd, cb, S, g, t);
-#pragma unroll
-        for(int n = 0; n < NT; ++n)
-#pragma unroll
-            for(int e = 0; e < 4; ++e)
-            {
-                Tp[(cb + 8 * n + 2 * t + (e & 1)) * kTrtriLdT + rb + g + (e >> 1) * 8] = acc[n][e];
-                acc[n][e] = 0.0;
-            }
-        __syncthreads();
-        // X21 = -X22 Tp, over L21: X22's row r ends at column r
-        trtri_mma<NT>(acc, X22 + rb, kTrtriLd, Tp + cb * kTrtriLdT, kTrtriLdT, 0, rb + 16, g, t);
-#pragma unroll
-        for(int n = 0; n < NT; ++n)
-#pragma unroll
-            for(int e = 0; e < 4; ++e)
-                L21[(cb + 8 * n + 2 * t + (e & 1)) * kTrtriLd + rb + g + (e >> 1) * 8] = -acc[n][e];
-        __syncthreads();
-    };
-    doubling(std::integral_constant<int, 16>{}, std::integral_constant<int, 1>{}, warp >> 1, 0, (warp & 1) * 8);
-    doubling(std::integral_constant<int, 32>{}, std::integral_constant<int, 2>{}, warp >> 2, (warp & 1) * 16,
-             (warp & 2) * 8);
-    // warps w and w + 4 share a scheduler: opposite row blocks give it even work in both products
-    doubling(std::integral_constant<int, 64>{}, std::integral_constant<int, 4>{}, 0,
-             (warp < 4 ? warp : 7 - warp) * 16, (warp >> 2) * 32);
+    // unit diagonals and padding are staged as 0, which like a zero diagonal entry is read as 1
+    trtri_invert(X, Tm, true);
 
     // ---- write inv(A_block) (bs x bs, ld = ldinv), zeros in the opposite triangle ----
     T* const out0 = p.upper ? out + (int64_t)(bs - 1) * (p.ldinv + 1) : out;

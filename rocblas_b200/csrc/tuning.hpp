@@ -51,7 +51,7 @@ struct Tuning
                                      // cycles (2^31: about a second), records error 4, returns
     int trsv_flag_min_n      = 256;  // trsv of one real vector: the flag-synchronised solve from
                                      // this order up
-    int trsv_flag_nb         = 128;  // ... its block rows (64 or 128)
+    int trsv_flag_nb         = 128;  // ... its block rows: 128 (streaming solve), 64 (flag solve)
     int crt_group_m          = 8;    // residue GEMM tile order: row tiles per group
     int crt_pair             = 1;    // residue GEMM as CTA pairs (cta_group::2, 256 x 256 tiles)
                                      // when it has every SM of the device

@@ -1,0 +1,76 @@
+"""The streaming TRSV (trsv_stream.cuh) at the edges of its 128-row blocks, all combinations, both
+element types, increments and leading dimensions, against the oracle; the flag solve in a workspace
+that holds only its flags gives the same answer; a wait that runs out is reported."""
+import ctypes
+import itertools
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import oracle  # noqa: E402
+import rocblas_b200 as rb  # noqa: E402
+from rocblas_b200 import devmem as dm  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def _trsv(h, dtype, uplo, trans, diag, n, A, lda, b, incx):
+    L = rb.lib()
+    fn = L.rocblas_dtrsv if dtype == np.float64 else L.rocblas_strsv
+    dA = dm.to_device(A)
+    x = torch.full((1 + (n - 1) * incx,), float("nan"), dtype=dA.dtype, device="cuda")
+    x[::incx] = torch.from_numpy(b).cuda()
+    assert fn(h.value, rb.UPLO[uplo], rb.TRANS[trans], rb.DIAG[diag], n, ctypes.c_void_p(dA.data_ptr()), lda,
+              ctypes.c_void_p(x.data_ptr()), incx) == 0
+    torch.cuda.synchronize()
+    if incx > 1:
+        gaps = x.clone()
+        gaps[::incx] = float("nan")
+        assert torch.isnan(gaps).all()
+    return x[::incx].cpu().numpy()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n", [256, 257, 383, 384, 385, 1000])
+def test_block_edges(n, dtype):
+    with rb.Handle() as h, rb.Handle() as flags_only:
+        assert rb.lib().rocblas_set_device_memory_size(flags_only.value, 64) == 0
+        for i, (uplo, trans, diag) in enumerate(itertools.product("UL", "NT", "NU")):
+            lda, incx = n + i % 3, 1 + i % 2
+            A, B = oracle.nan_triangle_problem(i, "L", uplo, trans, diag, n, 1, lda, n, dtype)
+            b = np.ascontiguousarray(B[:, 0])
+            X = oracle.trsm("L", uplo, trans, diag, 1.0, A, B)[:, 0]
+            tol = oracle.trsm_tolerance(dtype, n) * max(1.0, np.abs(X).max())
+            for handle in (h, flags_only):
+                out = _trsv(handle, dtype, uplo, trans, diag, n, A, lda, b, incx)
+                assert np.abs(out - X).max() <= tol, (uplo, trans, diag)
+
+
+@pytest.mark.parametrize("trans", "NT")
+def test_more_blocks_than_ctas(trans):
+    n = 20000  # 157 blocks
+    g = torch.Generator(device="cuda").manual_seed(1)
+    A = (torch.rand(n, n, generator=g, device="cuda", dtype=torch.float64) * 2 - 1) / n
+    A.diagonal().copy_(1 + torch.rand(n, generator=g, device="cuda", dtype=torch.float64))
+    b = torch.rand(n, generator=g, device="cuda", dtype=torch.float64)
+    x = b.clone()
+    with rb.Handle() as h:
+        assert rb.lib().rocblas_dtrsv(h.value, rb.fill_lower, rb.TRANS[trans], rb.diagonal_non_unit, n,
+                                      ctypes.c_void_p(A.data_ptr()), n, ctypes.c_void_p(x.data_ptr()), 1) == 0
+        torch.cuda.synchronize()
+    M = torch.tril(A.mT)  # the stored lower triangle, as written
+    M = M if trans == "N" else M.mT
+    # residual of a backward stable solve: n eps of |M| |x|
+    assert ((M @ x - b).abs() <= 2.3e-16 * n * (M.abs() @ x.abs())).all()
+
+
+def test_non_finite_entry_reaches_only_its_own_and_later_rows():
+    n, row = 700, 300
+    A, B = oracle.nan_triangle_problem(3, "L", "L", "N", "N", n, 1, n, n, np.float64)
+    b = np.ascontiguousarray(B[:, 0])
+    b[row] = np.inf
+    with rb.Handle() as h:
+        out = _trsv(h, np.float64, "L", "N", "N", n, A, n, b, 1)
+    assert np.isfinite(out[:row]).all() and not np.isfinite(out[row:]).any()
