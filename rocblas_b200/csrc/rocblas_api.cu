@@ -258,6 +258,8 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
         }
     }
 
+    pr.chain_small = 1;
+    pr.chain_small = use_chain(pr);
     const size_t ws_bytes = trsm_workspace_bytes<T>(pr, have_invA);
     if(h->size_query)
         return ws_bytes ? h->set_optimal_size(ws_bytes) : rocblas_status_size_unchanged;
@@ -279,13 +281,18 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
             // a workspace too small for the flags of narrow strips may hold those of the widest
             pr.chain_w = 64;
             ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
-            if(!ws && std::is_same<T, float>::value)
+            if(!ws)
             {
-                pr.chain_w = -1; // the recursive solve needs no flags
-                ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
+                pr.chain_small = 0; // the strip solver, where it can take the order, needs none,
+                pr.chain_w     = 0;
+                if(choose_algo(pr) != Algo::block && std::is_same<T, float>::value)
+                {
+                    pr.chain_w = -1; // and the recursive FP32 solve no flags
+                    ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
+                }
             }
         }
-        if(!ws && !have_invA)
+        if(!ws && !have_invA && choose_algo(pr) != Algo::block)
         {
             // backup: recursive solve with block-solver leaves needs no workspace
             perf = rocblas_status_perf_degraded;

@@ -67,6 +67,7 @@ struct TrsmProblem
     int         crt_pair_ok = 0; // the residue GEMM may run as CTA pairs on sm_count SMs that
                                  // are whole SM pairs (set beside a kernel placed in pairs)
     int         chain_w = 0; // strip width of the chain solve (0: chain_width's choice; < 0: no chain)
+    int         chain_small = 0; // orders the strip solver could take may go to the chain (choose_algo)
     int         k() const { return side_left ? m : n; }
     // op(A) lower?
     int oplower() const { return (!upper) != (trans != 0); }
@@ -358,6 +359,11 @@ static Algo choose_algo(const TrsmProblem<T>& pr)
         return Algo::recursive;
     if(k <= t.block_always_k)
         return Algo::block;
+    // One system with many strips: above 256 rows the chain's four MMA warps more per SM and its
+    // levels beat the strip solver's one CTA per strip (512 x 2048: 67 against 112 us, 512 x 8192
+    // 140 against 151, 300 x 4096 the same), below it they do not (256 x 4096: 52 against 43).
+    if(pr.chain_small && pr.batch == 1 && k > 256)
+        return Algo::recursive;
     const int64_t ncols   = pr.side_left ? pr.n : pr.m;
     const int64_t nstrips = ceil_div(ncols, kBsW) * (int64_t)pr.batch;
     return nstrips * 100 >= (int64_t)pr.sm_count * t.block_min_strips_pct ? Algo::block

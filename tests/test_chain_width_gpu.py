@@ -108,3 +108,20 @@ def test_fp32_with_many_columns(k, cols, fixed):
         out = _solve(h, "L", "L", "N", "N", k, cols, A, B)  # status success
     X = oracle.trsm("L", "L", "N", "N", 1.25, A, B)
     assert oracle.matrix_norm_1(X, out) <= oracle.trsm_tolerance(np.float32, k)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("k,cols", [(257, 2000), (512, 1300), (256, 2000)])
+@pytest.mark.parametrize("fixed", [False, True])
+def test_small_orders_with_many_columns(k, cols, dtype, fixed):
+    """Orders above 256 go to the chain; in a workspace that holds nothing, to the strip solver,
+    with the same status."""
+    for side, uplo in ("LL", "RU"):
+        m, n = (k, cols) if side == "L" else (cols, k)
+        A, B = oracle.nan_triangle_problem(k, side, uplo, "N", "N", m, n, k, m, dtype)
+        with rb.Handle() as h:
+            if fixed:
+                assert rb.lib().rocblas_set_device_memory_size(h.value, 64) == 0
+            out = _solve(h, side, uplo, "N", "N", m, n, A, B)
+        X = oracle.trsm(side, uplo, "N", "N", 1.25, A, B)
+        assert oracle.matrix_norm_1(X, out) <= oracle.trsm_tolerance(dtype, max(m, n))
