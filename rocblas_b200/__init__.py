@@ -30,7 +30,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
     "-shared",
 ]
-SOURCES = ["rocblas_api.cu", "chain_kernels.cu", "tile_kernels.cu"]
+SOURCES = ["rocblas_api.cu", "chain_kernels.cu", "chain_kernels_complex.cu", "tile_kernels.cu"]
 
 # ---- enums (include/rocblas.h; library/include/internal/rocblas-types.h:123-234) ---------
 operation_none, operation_transpose, operation_conjugate_transpose = 111, 112, 113

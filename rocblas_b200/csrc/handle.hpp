@@ -73,6 +73,10 @@ struct _rocblas_handle
     // Borrow `bytes` of workspace for the duration of one call; nullptr if not available.
     void* borrow(size_t bytes);
 
+    // As borrow, for a path that has another one needing less: while the stream is being captured
+    // managed memory is not grown (that allocates).
+    void* borrow_optional(size_t bytes);
+
     // release the managed allocation (not a user buffer)
     rocblas_status free_mem();
 };

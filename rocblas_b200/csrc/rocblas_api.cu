@@ -59,6 +59,20 @@ void* _rocblas_handle::borrow(size_t bytes)
     return mem;
 }
 
+void* _rocblas_handle::borrow_optional(size_t bytes)
+{
+    if(owner == MemOwner::managed && roundup(bytes) > mem_size)
+    {
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if(cudaStreamIsCapturing(stream, &capturing) != cudaSuccess)
+            cudaGetLastError(); // the legacy stream beside another stream's capture
+        else if(capturing == cudaStreamCaptureStatusNone)
+            return borrow(bytes);
+        return nullptr;
+    }
+    return borrow(bytes);
+}
+
 rocblas_status _rocblas_handle::free_mem()
 {
     if(mem && owner != MemOwner::user_owned)
@@ -275,24 +289,36 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
     void* ws = nullptr;
     if(ws_bytes)
     {
-        ws = h->borrow(ws_bytes);
+        ws = h->borrow_optional(ws_bytes);
         if(!ws && use_chain(pr))
         {
-            // a workspace too small for the flags of narrow strips may hold those of the widest
-            pr.chain_w = 64;
-            ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
-            if(!ws)
+            // a workspace too small for this path: the strip solver, where it can take the order,
+            // and the complex recursion need none; the flags of the widest strips take least; the
+            // recursive FP32 solve needs no flags
+            TrsmProblem<T> small = pr;
+            small.chain_small    = 0;
+            if(is_cplx<T>::value || choose_algo(small) == Algo::block)
             {
-                pr.chain_small = 0; // the strip solver, where it can take the order, needs none,
-                pr.chain_w     = 0;
-                if(choose_algo(pr) != Algo::block && std::is_same<T, float>::value)
+                pr.chain_small = 0;
+                pr.chain_w     = is_cplx<T>::value ? -1 : 0;
+            }
+            else
+            {
+                const bool recursive = std::is_same<T, float>::value
+                                       && (pr.side_left ? pr.n : pr.m) > tuning().chain_max_cols_f32;
+                pr.chain_w = 64;
+                ws         = recursive ? h->borrow_optional(trsm_workspace_bytes<T>(pr, have_invA))
+                                       : h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
+                if(!ws && recursive)
                 {
-                    pr.chain_w = -1; // and the recursive FP32 solve no flags
+                    pr.chain_w = -1;
                     ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
                 }
             }
         }
-        if(!ws && !have_invA && choose_algo(pr) != Algo::block)
+        else if(!ws)
+            ws = h->borrow(ws_bytes);
+        if(!ws && !have_invA && !is_cplx<T>::value && choose_algo(pr) != Algo::block)
         {
             // backup: recursive solve with block-solver leaves needs no workspace
             perf = rocblas_status_perf_degraded;
@@ -593,7 +619,7 @@ rocblas_status trsv_impl(rocblas_handle h, rocblas_fill uplo, rocblas_operation 
             if((st = device_ready(h)) != rocblas_status_success)
                 return st;
             int*  err = ensure_err(h);
-            void* ws  = h->borrow(bytes);
+            void* ws  = stream ? h->borrow_optional(bytes) : h->borrow(bytes);
             if(stream && (!ws || reinterpret_cast<uintptr_t>(ws) % 16)) // the pairs are 16-byte accesses
             {
                 stream = false;

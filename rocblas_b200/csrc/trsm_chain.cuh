@@ -38,7 +38,9 @@
 // records error code 4, all roles run out without waiting, and the CTA stops, so a wrong flag
 // cannot hang the GPU.
 // FP32 systems are staged as FP32 and computed in FP64 (the DMMA path is the one this kernel
-// has); the result is rounded to FP32 once.
+// has); the result is rounded to FP32 once.  Complex systems run as real ones of twice the order
+// (ChainReal): ztrsm 2048 x 1000, which recursed over one-CTA leaves, 2.30 -> 0.84 ms, and 8192 x
+// 2048 25.4 -> 17.9 ms.
 //
 // The 16 side/uplo/trans/diag cases use the index map of block_solve.cuh: side L solves
 // M Y = alpha C with M = op(A), C = B; side R solves M Y = alpha C with M = op(A)^T, C = B^T;
@@ -104,6 +106,7 @@ struct ChainParams
     // device by chain_vb_prepass_kernel
     const ChainVbHeader<T>* vhdr;
     Scalar<T>      alpha;   // the caller's alpha
+    int            conj = 0; // complex: M's entries are conjugated
     int            first;   // 1: this solve applies alpha; 0: it applies 1 (a sub-solve after an update)
     int*           flags;   // one per item id, zero at launch
     int*           counter; // 8-byte claim counter, zero at launch
@@ -133,6 +136,24 @@ __device__ __forceinline__ void chain_cp_async(uint32_t smem, const T* gmem, boo
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem), "l"(gmem), "r"(n) : "memory");
 }
 
+// Storage of one real number of T, and whether T is complex.  A complex system is solved as the
+// real one of twice the order whose matrix holds [[re, -im], [im, re]] for every entry (rows and
+// columns interleaved): C's interleaved storage is then the real right-hand sides as it stands,
+// a block of 128 rows is one of 64 complex rows, and the chunks of M keep the complex entries, of
+// which a lane reads the component that its row's and column's parity select, with a sign.
+template <typename T>
+struct ChainReal
+{
+    using type = T;
+    static constexpr int parts = 1;
+};
+template <typename R>
+struct ChainReal<cplx<R>>
+{
+    using type = R;
+    static constexpr int parts = 2;
+};
+
 // Shared memory: a ring of stages, each a chunk of M (128 rows o x kBK columns k) and of X (kBK x
 // W), then the tile T (128 x W doubles).  Layouts: M [k][o] (KCP = false) or [o][k] (KCP), X
 // [k][n] (KCQ = false) or [n][k] (KCQ), elements of type T.  Row pitches keep the fragment reads
@@ -141,13 +162,15 @@ __device__ __forceinline__ void chain_cp_async(uint32_t smem, const T* gmem, boo
 // Chunks are 32 deep where four stages fit in shared memory (narrow strips, whose wait for a block
 // is covered by the whole tile of M and the start of the inverse in the ring), else 16 deep;
 // either depth divides the 128-row blocks, so a chunk never spans two blocks.
-template <typename T, int W, bool KCP, bool KCQ>
+template <typename TT, int W, bool KCP, bool KCQ>
 struct ChainCfg
 {
+    using T = typename ChainReal<TT>::type;
+    static constexpr int kParts = ChainReal<TT>::parts; // reals per entry of M
     static constexpr int slow_pitch(int n) { return sizeof(T) == 8 ? n + 4 : n + (n % 32 == 0 || n % 32 == 16 ? 8 : 0); }
     static constexpr int pitch_p(int bk) { return KCP ? bk + 4 : slow_pitch(kChainNB); }
     static constexpr int pitch_q(int bk) { return KCQ ? bk + 4 : slow_pitch(W); }
-    static constexpr int stage_p(int bk) { return KCP ? kChainNB * pitch_p(bk) : bk * pitch_p(bk); }
+    static constexpr int stage_p(int bk) { return (KCP ? kChainNB : bk) / kParts * pitch_p(bk); }
     static constexpr int stage_q(int bk) { return KCQ ? W * pitch_q(bk) : bk * pitch_q(bk); }
     static constexpr size_t kBytesT = sizeof(double) * (size_t)kChainNB * (W + 4);
     static constexpr size_t kRoom   = 226 * 1024 - kBytesT; // for the ring; the barriers take the rest
@@ -176,7 +199,7 @@ struct ChainCfg
     static constexpr int kSplit = TM * TN == 1 ? 4 : TM * TN == 2 ? 2 : 1;
 };
 
-// One claimed item, resolved for all roles.
+// One claimed item, resolved for all roles; rows, sizes and leading dimensions in reals.
 template <typename T>
 struct ChainItem
 {
@@ -194,10 +217,13 @@ struct ChainItem
 
 // W right-hand sides per item (8, 16, 32 or 64).  KCP: M's K index is contiguous in memory (tM);
 // KCQ: C's row index is contiguous (side L).  VB: the variable-size tables of p describe the items.
-template <typename T, int W, bool KCP, bool KCQ, bool VB>
-__global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParams<T> p)
+template <typename TT, int W, bool KCP, bool KCQ, bool VB>
+__global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParams<TT> p)
 {
-    using Cfg = ChainCfg<T, W, KCP, KCQ>;
+    using Cfg = ChainCfg<TT, W, KCP, KCQ>;
+    using T   = typename Cfg::T;
+    constexpr int  PT = Cfg::kParts;
+    constexpr bool CX = PT == 2;
     constexpr int TM = Cfg::TM, TN = Cfg::TN, BK = Cfg::kBK, NS = Cfg::kStages, SP = Cfg::kSplit;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T*      ring = reinterpret_cast<T*>(smem_raw);
@@ -248,13 +274,25 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
 
     // alpha == 0 anywhere in the call means B := 0 with A unreferenced, also for sub-solves
     // that would otherwise apply 1
-    const double ua    = (double)p.alpha.get();
-    const double alpha = ua == 0.0 ? 0.0 : (p.first ? ua : 1.0);
-    const bool   zero  = alpha == 0.0;
+    double alpha, alpha_i = 0.0;
+    if constexpr(CX)
+    {
+        const TT ua = p.alpha.get();
+        alpha   = (double)ua.x;
+        alpha_i = (double)ua.y;
+    }
+    else
+        alpha = (double)p.alpha.get();
+    const bool zero = alpha == 0.0 && alpha_i == 0.0;
+    if(!zero && !p.first)
+    {
+        alpha   = 1.0;
+        alpha_i = 0.0;
+    }
 
     // claim the next item (one thread)
     auto claim = [&](ChainItem<T>& q) {
-        ChainVbHeader<T> H{};
+        ChainVbHeader<TT> H{};
         if constexpr(VB)
             H = *p.vhdr;
         const int64_t total = VB ? (H.maxnb > 0 ? H.vL[H.maxnb] : 0) : p.items;
@@ -270,6 +308,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
         T*       B;
         if constexpr(VB)
         {
+            static_assert(!CX || !VB, "variable batches are real");
             // level: last j with vL[j] <= item; system: last i < vcnt[j] with vP[i] <= r
             int lo = 0, hi = H.maxnb - 1;
             while(lo < hi)
@@ -292,7 +331,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                     z = mid - 1;
             }
             strip = r - H.vP[a];
-            const ChainSys<T> v = H.vsys[a];
+            const ChainSys<TT> v = H.vsys[a];
             A = v.A; q.inv = v.invA; B = v.B; q.lda = v.lda; q.ldb = v.ldb;
             k = v.k; ncols = v.ncols; q.nb = v.nb; q.forward = v.forward;
             q.flag0   = H.flags + H.vP[a] + strip;
@@ -304,8 +343,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
             const int64_t js   = item / p.ns;
             const int     sysi = (int)(js % p.systems);
             j = (int)(js / p.systems);
-            A = p.A.get(sysi); q.inv = p.invA.get(sysi); B = p.B.get(sysi);
-            q.lda = p.lda; q.ldb = p.ldb; k = p.k; ncols = p.ncols; q.nb = p.nb;
+            A     = reinterpret_cast<const T*>(p.A.get(sysi));
+            q.inv = reinterpret_cast<const T*>(p.invA.get(sysi));
+            B     = reinterpret_cast<T*>(p.B.get(sysi));
+            q.lda = p.lda * PT; q.ldb = p.ldb * PT; k = p.k * PT; ncols = p.ncols; q.nb = p.nb;
             q.forward = p.forward;
             q.flag0   = p.flags + (int64_t)sysi * p.ns + strip;
             q.fstride = (int64_t)p.systems * p.ns;
@@ -315,9 +356,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
         q.r0   = b * kChainNB;
         q.bs   = min(kChainNB, k - q.r0);
         q.wv   = min(W, ncols - strip * W);
-        q.M    = KCP ? A + (int64_t)q.r0 * q.lda : A + q.r0;
-        q.inv += (int64_t)b * kChainNB * kChainNB;
-        q.C    = KCQ ? B + (int64_t)strip * W * q.ldb : B + strip * W;
+        q.M    = KCP ? A + (int64_t)(q.r0 / PT) * q.lda : A + q.r0;
+        q.inv += (int64_t)b * kChainNB * kChainNB / PT;
+        q.C    = KCQ ? B + (int64_t)strip * W * q.ldb : B + strip * W * PT;
         // K rows of the finished blocks: forward [0, r0) ascending; backward [r0 + bs, k)
         // descending, in chunks of BK rows aligned to multiples of BK (never across a block)
         q.klo  = q.forward ? 0 : q.r0 + q.bs;
@@ -379,11 +420,12 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                 // ---- chunks of M, then of the inverse --------------------
                 // A warp copies every third line of a chunk: a K column (128 rows; four copies
                 // per lane) or, K contiguous, 32 / BK rows of BK columns.
-                constexpr int kLines = KCP ? kChainNB * BK / 32 : BK;
+                // (complex: half as many lines, of the same number of reals)
+                constexpr int kLines = (KCP ? kChainNB * BK / 32 : BK) / PT;
                 constexpr int kPer   = KCP ? 1 : kChainNB / 32; // copies per lane and line
                 const int     cw  = warp - kChainMmaWarps;
                 const int     o0  = KCP ? lane / BK : lane, kk0 = KCP ? lane % BK : 0;
-                constexpr int kLineO = KCP ? 32 / BK : 0, kLineK = KCP ? 0 : 1;
+                constexpr int kLineO = KCP ? 32 / BK : 0;
                 constexpr uint32_t kDstLine = (uint32_t)sizeof(T) * (KCP ? kLineO : 1) * Cfg::kPitchP;
                 const uint32_t dst0 = smem_u32(ring) + (uint32_t)sizeof(T) * (KCP ? o0 * Cfg::kPitchP + kk0 : o0)
                                       + cw * kDstLine;
@@ -393,7 +435,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                     const int k0 = q.forward ? i * BK : q.ktop - (i + 1) * BK;
                     slot();
                     uint32_t dst = dst0 + st * (uint32_t)(sizeof(T) * Cfg::kStage);
-                    const T* src = (KCP ? q.M + (k0 + kk0) + (int64_t)o0 * q.lda : q.M + o0 + (int64_t)k0 * q.lda)
+                    const T* src = (KCP ? q.M + (k0 + kk0) + (int64_t)o0 * q.lda : q.M + o0 + (int64_t)(k0 / PT) * q.lda)
                                    + cw * line;
                     const bool whole = q.bs == kChainNB && k0 + BK <= q.khi;
                     if(whole)
@@ -416,7 +458,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
 #pragma unroll
                             for(int u = 0; u < kPer; ++u)
                             {
-                                const bool valid = o0 + e * kLineO + u * 32 < q.bs && k0 + kk0 + e * kLineK < q.khi;
+                                const bool valid = KCP ? (o0 + e * kLineO) * PT < q.bs && k0 + kk0 < q.khi
+                                                       : o0 + u * 32 < q.bs && k0 + e * PT < q.khi;
                                 chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), valid ? src + u * 32 : q.M, valid);
                             }
                             dst += kChainCopyWarps * kDstLine;
@@ -437,7 +480,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                     if(q.bs == kChainNB)
                     {
                         constexpr int kLine = (KCP ? kLineO : 1) * kChainNB;
-                        const T* src = (KCP ? q.inv + (k0 + kk0) + o0 * kChainNB : q.inv + o0 + k0 * kChainNB) + cw * kLine;
+                        const T* src = (KCP ? q.inv + (k0 + kk0) + o0 * kChainNB : q.inv + o0 + k0 / PT * kChainNB) + cw * kLine;
 #pragma unroll 4
                         for(int e = cw; e < kLines; e += kChainCopyWarps)
                         {
@@ -455,10 +498,11 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
 #pragma unroll
                         for(int u = 0; u < kPer; ++u)
                         {
-                            const int  o = o0 + e * kLineO + u * 32, kr = k0 + kk0 + e * kLineK;
-                            const bool valid = o < q.bs && kr < q.bs;
-                            chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T),
-                                              valid ? q.inv + (KCP ? kr + o * kChainNB : o + kr * kChainNB) : q.inv, valid);
+                            const bool valid = KCP ? (o0 + e * kLineO) * PT < q.bs && k0 + kk0 < q.bs
+                                                   : o0 + u * 32 < q.bs && k0 + e * PT < q.bs;
+                            const T*   src   = KCP ? q.inv + (k0 + kk0) + (o0 + e * kLineO) * kChainNB
+                                                   : q.inv + (o0 + u * 32) + (k0 / PT + e) * kChainNB;
+                            chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), valid ? src : q.inv, valid);
                         }
                         dst += kChainCopyWarps * kDstLine;
                     }
@@ -477,8 +521,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                 const int     f0 = lane % kLanes, l0 = lane / kLanes;
                 const uint32_t dst0 = smem_u32(ring)
                                       + (uint32_t)sizeof(T) * (Cfg::kStageP + l0 * Cfg::kPitchQ + f0);
-                const T* const src0 = q.C + f0 + l0 * q.ldb;
-                const int64_t  line = kStep * q.ldb;
+                // a complex strip from the right has its two components as two K lines
+                const T* const src0 = q.C + f0 * (KCQ ? 1 : PT);
+                auto line_of = [&](int l) -> int64_t { return KCQ || !CX ? l * q.ldb : (l >> 1) * q.ldb + (l & 1); };
+                constexpr int kFastStep = KCQ ? 32 : 32 * PT;
                 constexpr uint32_t kDstLine = (uint32_t)sizeof(T) * kStep * Cfg::kPitchQ;
                 // solve positions [0, done) of the item's nprev earlier ones are known finished; one
                 // round of loads looks at the next 32 flags, so finished blocks cost no round trip each
@@ -517,25 +563,29 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                         __syncwarp(); // the lanes' acquires order the warp's copies of X below
                     }
                     uint32_t dst = dst0 + st * (uint32_t)(sizeof(T) * Cfg::kStage);
-                    const T* src = src0 + (KCQ ? k0 : k0 * q.ldb);
+                    const T* base = src0 + (KCQ ? k0 : line_of(k0));
                     if(q.wv == W && k0 + BK <= q.khi)
                     {
 #pragma unroll 8
-                        for(int e = 0; e < kLines; e += kStep, src += line, dst += kDstLine)
+                        for(int e = 0; e < kLines; e += kStep, dst += kDstLine)
+                        {
+                            const T* src = base + line_of(l0 + e);
 #pragma unroll
                             for(int u = 0; u < kRep; ++u)
-                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), src + u * 32, true);
+                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), src + u * kFastStep, true);
+                        }
                     }
                     else
                     {
 #pragma unroll 1
-                        for(int e = 0; e < kLines; e += kStep, src += line, dst += kDstLine)
+                        for(int e = 0; e < kLines; e += kStep, dst += kDstLine)
 #pragma unroll
                             for(int u = 0; u < kRep; ++u)
                             {
                                 const int  f = f0 + u * 32, l = l0 + e;
                                 const bool valid = (KCQ ? l : f) < q.wv && k0 + (KCQ ? f : l) < q.khi;
-                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T), valid ? src + u * 32 : q.C, valid);
+                                chain_cp_async<T>(dst + u * 32 * (uint32_t)sizeof(T),
+                                                  valid ? base + line_of(l) + u * kFastStep : q.C, valid);
                             }
                     }
                     mbar_arrive_cp_async(&full[st]);
@@ -572,7 +622,17 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
             ph ^= 1;
         }
     };
+    // complex: rows o have the parity of g and columns kk that of t, which fixes the component and
+    // its sign for the lane
+    const int  part = (g ^ t) & 1;
+    const bool flip = CX && part && ((g & 1) == 0) != (p.conj != 0);
     auto ldP = [&](const T* sP, int o, int kk) -> double {
+        if constexpr(CX)
+        {
+            const double v = (double)(KCP ? sP[(o >> 1) * Cfg::kPitchP + (kk & ~1) + part]
+                                          : sP[(kk >> 1) * Cfg::kPitchP + (o & ~1) + part]);
+            return __hiloint2double(__double2hiint(v) ^ (flip ? 0x80000000 : 0), __double2loint(v));
+        }
         return (double)(KCP ? sP[o * Cfg::kPitchP + kk] : sP[kk * Cfg::kPitchP + o]);
     };
     auto ldQ = [&](const T* sQ, int n, int kk) -> double {
@@ -600,7 +660,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
             break;
         // C(r0 + o, col) of this thread's output (i, jn, e)
         auto caddr = [&](int o, int col) -> T* {
-            return KCQ ? q.C + (q.r0 + o) + (int64_t)col * q.ldb : q.C + col + (int64_t)(q.r0 + o) * q.ldb;
+            const int r = q.r0 + o;
+            return KCQ  ? q.C + r + (int64_t)col * q.ldb
+                   : CX ? q.C + 2 * col + (int64_t)(r >> 1) * q.ldb + (r & 1)
+                        : q.C + col + (int64_t)r * q.ldb;
         };
         auto out_o = [&](int i, int e) { return row0 + i * 16 + g + (e >> 1) * 8; };
         auto out_n = [&](int jn, int e) { return col0 + jn * 8 + 2 * t + (e & 1); };
@@ -617,7 +680,14 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                 for(int e = 0; e < 4; ++e)
                 {
                     const int o = out_o(i, e), col = out_n(jn, e);
-                    c[jn][e] = !zero && o < q.bs && col < q.wv ? alpha * (double)__ldcg(caddr(o, col)) : 0.0;
+                    c[jn][e] = 0.0;
+                    if(!zero && o < q.bs && col < q.wv)
+                    {
+                        const T* src = caddr(o, col);
+                        c[jn][e]     = alpha * (double)__ldcg(src);
+                        if constexpr(CX) // the other component, times i alpha_i
+                            c[jn][e] += (o & 1 ? alpha_i : -alpha_i) * (double)__ldcg(o & 1 ? src - 1 : src + 1);
+                    }
                 }
         };
         double acc[SP][TM][TN][4], cv[TM][TN][4];
@@ -742,7 +812,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                         for(int e = 0; e < 4; ++e)
                         {
                             const int o = out_o(i, 2 * (e & 1)), kr = kb + t + 4 * (e >> 1);
-                            if(q.forward ? kr > o : kr < o)
+                            if(q.forward ? kr / PT > o / PT : kr / PT < o / PT)
                                 fa[i][e] = 0.0;
                         }
 #pragma unroll
@@ -828,7 +898,7 @@ static void launch_chain_cfg(const ChainParams<T>& p, int sms, int64_t max_items
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kChainThreads, Cfg::kSmem);
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(max_items, (int64_t)sms * std::max(per_sm, 1)));
     // algorithmic work (uniform batch): k * k * ncols per system, the trsm flop count
-    const double work = VB ? 0.0 : (double)p.systems * p.k * (double)p.k * p.ncols;
+    const double work = VB ? 0.0 : (is_cplx<T>::value ? 4.0 : 1.0) * p.systems * p.k * (double)p.k * p.ncols;
     TimedLaunch tl(KernelClass::chain, s, work);
     if(cluster2 && grid % 2 == 0)
     {
@@ -878,4 +948,12 @@ extern template void launch_chain_w<float, 64, false>(const ChainParams<float>&,
 extern template void launch_chain_w<float, 32, true>(const ChainParams<float>&, bool, bool, int, int64_t, cudaStream_t, bool);
 extern template void launch_chain_w<float, 64, true>(const ChainParams<float>&, bool, bool, int, int64_t, cudaStream_t, bool);
 
+extern template void launch_chain_w<cplx<double>, 8, false>(const ChainParams<cplx<double>>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<cplx<double>, 16, false>(const ChainParams<cplx<double>>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<cplx<double>, 32, false>(const ChainParams<cplx<double>>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<cplx<double>, 64, false>(const ChainParams<cplx<double>>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<cplx<float>, 8, false>(const ChainParams<cplx<float>>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<cplx<float>, 16, false>(const ChainParams<cplx<float>>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<cplx<float>, 32, false>(const ChainParams<cplx<float>>&, bool, bool, int, int64_t, cudaStream_t, bool);
+extern template void launch_chain_w<cplx<float>, 64, false>(const ChainParams<cplx<float>>&, bool, bool, int, int64_t, cudaStream_t, bool);
 } // namespace rb200

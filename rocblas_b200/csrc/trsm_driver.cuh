@@ -16,8 +16,9 @@
 //     Without workspace for invA the leaves use the block solver instead and the call
 //     reports rocblas_status_perf_degraded, as the reference's backup path does
 //     (rocblas_trsm_kernels.hpp:1926-1944).
-//   * complex types: the same recursion with block-solver leaves (no invA) and the complex
-//     DMMA tiles (gemm_cdmma.cuh) for the updates; trans C conjugates A in both.
+//   * complex types: the chain on inverses of 64-row blocks (one system), else the same recursion
+//     with block-solver leaves (no invA) and the complex DMMA tiles (gemm_cdmma.cuh) for the
+//     updates; trans C conjugates A in both.
 #pragma once
 #include <algorithm>
 #include <atomic>
@@ -344,6 +345,44 @@ static void build_invA(const TrsmProblem<T>& pr, BatchPtr<T> inv)
     launch_trtri<T>(t, (int)ceil_div(k, kInvNB), pr.batch, pr.stream);
 }
 
+// Inverses of a complex A's diagonal blocks of kCplxNB rows (ld kCplxNB), for the chain: the block
+// solver on identities, all blocks in one launch.
+constexpr int kCplxNB = kInvNB / 2;
+
+template <typename T>
+__global__ void identity_blocks_kernel(T* inv, int k)
+{
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if(i < (int64_t)k * kCplxNB)
+        inv[i] = i % kCplxNB == i / kCplxNB % kCplxNB ? T(1) : T(0);
+}
+
+template <typename T>
+static void build_cplx_inverses(const TrsmProblem<T>& pr, BatchPtr<T> inv)
+{
+    const int     k     = pr.k();
+    const int64_t total = (int64_t)k * kCplxNB;
+    identity_blocks_kernel<T><<<(unsigned)ceil_div(total, 256), 256, 0, pr.stream>>>(inv.base, k);
+    count_launch();
+    TrsmProblem<T> q = pr;
+    q.side_left = 1;
+    q.trans = q.conj = 0;
+    q.alpha = Scalar<T>{};
+    q.ldb   = kCplxNB;
+    q.batch = k / kCplxNB;
+    BatchPtr<T> A = pr.A, X = inv;
+    A.stride = (int64_t)kCplxNB * (pr.lda + 1);
+    X.stride = (int64_t)kCplxNB * kCplxNB;
+    if(q.batch)
+        launch_block_solve<T>(q, kCplxNB, kCplxNB, A, X, 1);
+    if(const int rem = k % kCplxNB)
+    {
+        const int64_t b = q.batch;
+        q.batch = 1;
+        launch_block_solve<T>(q, rem, rem, A.shifted(b * A.stride), X.shifted(b * X.stride), 1);
+    }
+}
+
 enum class Algo
 {
     block,
@@ -362,7 +401,9 @@ static Algo choose_algo(const TrsmProblem<T>& pr)
     // One system with many strips: above 256 rows the chain's four MMA warps more per SM and its
     // levels beat the strip solver's one CTA per strip (512 x 2048: 67 against 112 us, 512 x 8192
     // 140 against 151, 300 x 4096 the same), below it they do not (256 x 4096: 52 against 43).
-    if(pr.chain_small && pr.batch == 1 && k > 256)
+    // Complex strips are solved by a slower one-CTA solver (256 x 2000: 201 against 87 us on the
+    // chain, 129 against 81 in single precision; at 128 x 2000 75 against 67 and 53 against 58).
+    if(pr.chain_small && pr.batch == 1 && k > (is_cplx<T>::value ? 128 : 256))
         return Algo::recursive;
     const int64_t ncols   = pr.side_left ? pr.n : pr.m;
     const int64_t nstrips = ceil_div(ncols, kBsW) * (int64_t)pr.batch;
@@ -391,12 +432,17 @@ static int64_t strsm_sliced_half(const TrsmProblem<T>& pr)
 // A solve of more than one 128-row block runs as one chain launch (trsm_chain.cuh) when invA is
 // available: FP64 with at most chain_max_cols right-hand sides, FP32 unless its updates are worth
 // the slice engine (or strsm_slices 0 asks for the FFMA recursion).
+// Complex: one system given by its address, on inverse blocks of kCplxNB rows.
 template <typename T>
 static bool use_chain(const TrsmProblem<T>& pr)
 {
-    if(is_cplx<T>::value || choose_algo(pr) != Algo::recursive || pr.chain_w < 0 || pr.k() <= kInvNB)
+    if(choose_algo(pr) != Algo::recursive || pr.chain_w < 0)
         return false;
     const int64_t ncols = pr.side_left ? pr.n : pr.m;
+    if(is_cplx<T>::value)
+        return pr.batch == 1 && !pr.A.arr && ncols <= tuning().chain_max_cols;
+    if(pr.k() <= kInvNB)
+        return false;
     if(std::is_same<T, float>::value)
         return ncols <= tuning().chain_max_cols_f32 || (tuning().strsm_slices > 0 && strsm_sliced_half(pr) == 0);
     return ncols <= tuning().chain_max_cols;
@@ -438,8 +484,9 @@ template <typename T>
 static ChainShape chain_shape_of(const TrsmProblem<T>& pr)
 {
     const int ncols = pr.side_left ? pr.n : pr.m;
-    const int w     = pr.chain_w > 0 ? pr.chain_w : chain_width(pr.k(), ncols, pr.batch, pr.sm_count);
-    return chain_shape(pr.k(), ncols, pr.batch, w);
+    const int k     = pr.k() * ChainReal<T>::parts; // real rows
+    const int w     = pr.chain_w > 0 ? pr.chain_w : chain_width(k, ncols, pr.batch, pr.sm_count);
+    return chain_shape(k, ncols, pr.batch, w);
 }
 
 __global__ void chain_set_counter_kernel(int* counter, int v)
@@ -455,16 +502,18 @@ template <typename T>
 static void launch_chain_sub(const TrsmProblem<T>& pr, int b0, int b1, int first, int w, void* ws,
                              bool cluster2)
 {
-    const int        r0    = b0 * kInvNB;
-    const int        kk    = std::min(b1 * kInvNB, pr.k()) - r0;
+    constexpr int    PT = ChainReal<T>::parts, NB = kInvNB / PT; // rows of an inverse block
+    const int        r0    = b0 * NB;
+    const int        kk    = std::min(b1 * NB, pr.k()) - r0;
     const int        ncols = pr.side_left ? pr.n : pr.m;
-    const ChainShape cs    = chain_shape(kk, ncols, pr.batch, w);
+    const ChainShape cs    = chain_shape(kk * PT, ncols, pr.batch, w);
     int*             flags = reinterpret_cast<int*>(ws);
     cudaMemsetAsync(flags, 0, chain_workspace_bytes(cs), pr.stream);
     ChainParams<T> c{};
     c.A       = pr.A.shifted(r0 + (int64_t)r0 * pr.lda);
     c.lda     = pr.lda;
-    c.invA    = pr.invA.shifted((int64_t)b0 * kInvNB * kInvNB);
+    c.invA    = pr.invA.shifted((int64_t)b0 * NB * NB);
+    c.conj    = pr.conj;
     c.B       = pr.B.shifted(pr.side_left ? (int64_t)r0 : (int64_t)r0 * pr.ldb);
     c.ldb     = pr.ldb;
     c.k       = kk;
@@ -509,8 +558,9 @@ static void launch_chain_sub(const TrsmProblem<T>& pr, int b0, int b1, int first
 template <typename T>
 static size_t trsm_invA_bytes(const TrsmProblem<T>& pr, bool have_supplied_invA)
 {
-    // complex solves use block-solver leaves and need no invA
-    if(is_cplx<T>::value || choose_algo(pr) != Algo::recursive || have_supplied_invA)
+    if(is_cplx<T>::value) // the chain's own blocks; the recursion uses block-solver leaves
+        return use_chain(pr) ? (size_t)kCplxNB * (size_t)pr.k() * sizeof(T) : 0;
+    if(choose_algo(pr) != Algo::recursive || have_supplied_invA)
         return 0;
     return (size_t)kInvNB * (size_t)pr.k() * sizeof(T) * (size_t)pr.batch;
 }
@@ -553,6 +603,15 @@ static void trsm_run(TrsmProblem<T> pr, void* ws, bool supplied_invA)
     if constexpr(is_cplx<T>::value)
     {
         pr.invA = BatchPtr<T>{};
+        if(ws && use_chain(pr))
+        {
+            pr.invA.base     = reinterpret_cast<T*>(ws);
+            const size_t off = (trsm_invA_bytes(pr, false) + 255) / 256 * 256;
+            build_cplx_inverses<T>(pr, pr.invA);
+            launch_chain_sub<T>(pr, 0, (int)ceil_div(k, kCplxNB), 1, chain_shape_of(pr).w,
+                                reinterpret_cast<char*>(ws) + off);
+            return;
+        }
     }
     else
     {

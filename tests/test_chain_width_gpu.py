@@ -125,3 +125,42 @@ def test_small_orders_with_many_columns(k, cols, dtype, fixed):
             out = _solve(h, side, uplo, "N", "N", m, n, A, B)
         X = oracle.trsm(side, uplo, "N", "N", 1.25, A, B)
         assert oracle.matrix_norm_1(X, out) <= oracle.trsm_tolerance(dtype, max(m, n))
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+@pytest.mark.parametrize("w", [0, 8, 16, 32, 64])
+def test_complex_widths(width, w, dtype):
+    """Complex systems as real ones of twice the order: blocks of 64, every side / uplo / trans."""
+    assert width(w) == 0
+    alpha = 0.5 - 1.25j
+    with rb.Handle() as h:
+        for i, (side, uplo, trans, diag) in enumerate(itertools.product("LR", "UL", "NTC", "NU")):
+            k, cols = [(129, 1), (191, w + 1), (256, 9), (257, 2 * w + 3), (320, 33)][i % 5]
+            m, n = (k, cols) if side == "L" else (cols, k)
+            A, B = oracle.nan_triangle_problem(i, side, uplo, trans, diag, m, n, k + i % 3, m + i % 2, dtype)
+            dA, dB = dm.to_device(A), dm.to_device(B)
+            dm.trsm(h, side, uplo, trans, diag, m, n, alpha, dA, A.shape[0], dB, B.shape[0], alpha_on_device=i % 2 == 1)
+            torch.cuda.synchronize()
+            out = dm.to_host(dB)
+            X = oracle.trsm(side, uplo, trans, diag, alpha, A, np.asfortranarray(B[:m]))
+            assert oracle.matrix_norm_1(X, out[:m]) <= oracle.trsm_tolerance(dtype, max(m, n)), (side, uplo, trans, diag)
+            assert np.isnan(out[m:]).all()
+
+
+def test_capture_of_a_call_whose_workspace_was_never_grown():
+    """Paths that want more workspace than their fallback must not allocate under capture: a fresh
+    handle's complex solve, an order of the strip solver and a TRSV whose flags fit are captured."""
+    for dtype, k, cols in ((np.complex128, 200, 20), (np.float64, 400, 2000)):
+        A, B = oracle.nan_triangle_problem(k, "L", "L", "N", "N", k, cols, k, k, dtype)
+        X = oracle.trsm("L", "L", "N", "N", 1.0, A, B)
+        s = torch.cuda.Stream()
+        with rb.Handle() as h, torch.cuda.stream(s):
+            h.set_stream(ctypes.c_void_p(s.cuda_stream))
+            dA, dB0 = dm.to_device(A), dm.to_device(B)
+            dB = dB0.clone()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=s):
+                dm.trsm(h, "L", "L", "N", "N", k, cols, 1.0, dA, k, dB, k)
+            graph.replay()
+            s.synchronize()
+            assert oracle.matrix_norm_1(X, dm.to_host(dB)) <= oracle.trsm_tolerance(dtype, max(k, cols))
