@@ -1229,7 +1229,7 @@ __global__ void vb_copy_invalid_kernel(const int* invalid, rocblas_int* out)
 
 static_assert(sizeof(VbProblem) == sizeof(rocblas_b200_trsm_problem), "descriptor layout");
 
-// Persistent strip-solver launch over one queue; shared memory sized for systems up to kmax.
+// Persistent strip-solver launch over one queue of systems up to kmax.
 template <typename T>
 void launch_vb_queue(rocblas_handle h, const VbParams<T>& p, int kmax)
 {
@@ -1245,19 +1245,15 @@ void launch_vb_queue(rocblas_handle h, const VbParams<T>& p, int kmax)
         count_launch();
         return;
     }
-    auto launch = [&](auto kern, size_t smem) {
-        cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSsThreads, smem);
-        per_sm = std::max(per_sm, 1);
-        TimedLaunch tl(KernelClass::strip, h->stream, 0.0);
-        kern<<<h->sm_count * per_sm, kSsThreads, smem, h->stream>>>(p);
-        count_launch();
-    };
-    if(kmax <= 64)
-        launch(vb_persistent_kernel<T, 8, 2, 5>, SsCfg<T, 8, 2>::kSmem);
-    else
-        launch(vb_persistent_kernel<T, 16, 2, 3>, SsCfg<T, 16, 2>::kSmem);
+    auto             kern = vb_persistent_kernel<T, kSsRT, kSsNS, kSsCtas>;
+    constexpr size_t smem = SsCfg<T, kSsRT, kSsNS>::kSmem;
+    cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSsThreads, smem);
+    per_sm = std::max(per_sm, 1);
+    TimedLaunch tl(KernelClass::strip, h->stream, 0.0);
+    kern<<<h->sm_count * per_sm, kSsThreads, smem, h->stream>>>(p);
+    count_launch();
 }
 
 template <typename T>

@@ -174,10 +174,8 @@ static void launch_block_solve(const TrsmProblem<T>& pr, int m, int n, BatchPtr<
     };
     if constexpr(is_cplx<T>::value)
         launch(block_solve_kernel<T>, kBsThreads, block_solve_smem_bytes<T>(p.k));
-    else if(p.k <= 64)
-        launch(strip_solve_kernel<T, 8, 2, 5>, kSsThreads, SsCfg<T, 8, 2>::kSmem);
     else
-        launch(strip_solve_kernel<T, 16, 2, 3>, kSsThreads, SsCfg<T, 16, 2>::kSmem);
+        launch(strip_solve_kernel<T, kSsRT, kSsNS, kSsCtas>, kSsThreads, SsCfg<T, kSsRT, kSsNS>::kSmem);
 }
 
 // ---- recursive blocked solve --------------------------------------------------------------
