@@ -310,7 +310,7 @@ ROCBLAS_EXPORT rocblas_status rocblas_b200_dtrsm_mixed(rocblas_handle    handle,
  *   X := precision-form solve of op(A) X = alpha B (or X op(A) = alpha B);
  *   test: `check_columns` evenly spaced right-hand sides (columns of B for side left, rows for
  *         side right) are also solved by the plain FP64 form, on a second stream and a few SMs
- *         of their own (tuning keys refine_check_sms, refine_check_pairs: 6 SMs held as SM
+ *         of their own (tuning keys refine_check_sms, refine_check_pairs: 4 SMs held as SM
  *         pairs) while the precision-form solve runs on the others; the test passes when, for
  *         each of them,
  *         ||x - x_fp64||_inf <= tolerance * ||x_fp64||_inf;

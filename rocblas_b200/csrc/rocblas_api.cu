@@ -293,8 +293,7 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
         if(!ws && use_chain(pr))
         {
             // a workspace too small for this path: the strip solver, where it can take the order,
-            // and the complex recursion need none; the flags of the widest strips take least; the
-            // recursive FP32 solve needs no flags
+            // and the complex recursion need none, the recursive FP32 solve no counts
             TrsmProblem<T> small = pr;
             small.chain_small    = 0;
             if(is_cplx<T>::value || choose_algo(small) == Algo::block)
@@ -304,16 +303,9 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
             }
             else
             {
-                const bool recursive = std::is_same<T, float>::value
-                                       && (pr.side_left ? pr.n : pr.m) > tuning().chain_max_cols_f32;
-                pr.chain_w = 64;
-                ws         = recursive ? h->borrow_optional(trsm_workspace_bytes<T>(pr, have_invA))
-                                       : h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
-                if(!ws && recursive)
-                {
+                if(std::is_same<T, float>::value && (pr.side_left ? pr.n : pr.m) > tuning().chain_max_cols_f32)
                     pr.chain_w = -1;
-                    ws         = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
-                }
+                ws = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
             }
         }
         else if(!ws)
@@ -1693,9 +1685,7 @@ struct MixedPlan
     size_t inv_bytes = 0, sl_bytes = 0, ch_bytes = 0, total = 0;
 };
 
-// chain_w 0: the width of mixed_chain_width; 64, whose flags take least, where the workspace is
-// too small for that
-MixedPlan mixed_plan(const TrsmProblem<double>& pr, int slices, int moduli, int chain_w = 0)
+MixedPlan mixed_plan(const TrsmProblem<double>& pr, int slices, int moduli)
 {
     MixedPlan p;
     p.recursive = choose_algo(pr) == Algo::recursive;
@@ -1703,8 +1693,8 @@ MixedPlan mixed_plan(const TrsmProblem<double>& pr, int slices, int moduli, int 
         return p;
     p.inv_bytes = align256((size_t)kInvNB * pr.k() * sizeof(double));
     p.sl_bytes  = mixed_slice_workspace_bytes(pr, slices, moduli);
-    p.chain_w   = chain_w ? chain_w : mixed_chain_width(pr);
-    p.ch_bytes  = mixed_chain_workspace_bytes(pr, p.chain_w);
+    p.chain_w   = mixed_chain_width(pr);
+    p.ch_bytes  = mixed_chain_workspace_bytes(pr);
     p.total     = p.inv_bytes + align256(p.sl_bytes) + align256(p.ch_bytes);
     return p;
 }
@@ -1781,7 +1771,7 @@ rocblas_status trsm_mixed_impl(rocblas_handle h, rocblas_side side, rocblas_fill
     pr.ldb = ldb;
     pr.stream   = h->stream;
     pr.sm_count = h->sm_count;
-    MixedPlan plan = mixed_plan(pr, slices, moduli);
+    const MixedPlan plan = mixed_plan(pr, slices, moduli);
     if(h->size_query)
         return plan.total ? h->set_optimal_size(plan.total) : rocblas_status_size_unchanged;
     if((st = device_ready(h)) != rocblas_status_success)
@@ -1792,11 +1782,6 @@ rocblas_status trsm_mixed_impl(rocblas_handle h, rocblas_side side, rocblas_fill
         pr.alpha.ptr = alpha;
     int*  err = plan.recursive ? ensure_err(h) : nullptr;
     void* ws  = plan.total ? h->borrow(plan.total) : nullptr;
-    if(plan.recursive && !ws)
-    {
-        plan = mixed_plan(pr, slices, moduli, 64);
-        ws   = h->borrow(plan.total);
-    }
     if(plan.recursive && (!ws || !err))
         return rocblas_status_memory_error;
     if(!mixed_run(pr, slices, moduli, plan, ws, err, true))
@@ -2018,7 +2003,7 @@ rocblas_status trsm_refined_impl(rocblas_handle h, rocblas_side side, rocblas_fi
     const int  nb_flag = (int)ceil_div(left ? m : n, 128);
     // workspace: the precision form's | B0 (m x n) | R (m x n) | the tested right-hand sides |
     // their chain flags | the test's maxima
-    MixedPlan       plan  = mixed_plan(pr, S, moduli);
+    const MixedPlan plan  = mixed_plan(pr, S, moduli);
     const size_t    mn    = (size_t)m * n * sizeof(double);
     const size_t    smp   = (size_t)srows * scols * sizeof(double);
     // the chain's strip width: that of the up to 8 tested columns, where refine_check_w allows it
@@ -2028,16 +2013,10 @@ rocblas_status trsm_refined_impl(rocblas_handle h, rocblas_side side, rocblas_fi
     const size_t    fl    = ps_flag    ? (size_t)nb_flag * 2 * sizeof(int)
                             : ps_chain ? chain_workspace_bytes(chain_shape(ps.k(), c, 1, ps_w))
                                        : 0;
-    size_t o_b0 = 0, o_r = 0, o_xs = 0, o_fl = 0, o_mx = 0, total = 0;
-    auto   lay_out = [&]() {
-        o_b0  = align256(plan.total);
-        o_r   = o_b0 + align256(mn);
-        o_xs  = o_r + (max_it > 0 ? align256(mn) : 0);
-        o_fl  = o_xs + align256(smp);
-        o_mx  = o_fl + align256(fl);
-        total = o_mx + align256(sizeof(double) * 2 * (size_t)c);
-    };
-    lay_out();
+    const size_t    o_b0  = align256(plan.total), o_r = o_b0 + align256(mn);
+    const size_t    o_xs  = o_r + (max_it > 0 ? align256(mn) : 0), o_fl = o_xs + align256(smp);
+    const size_t    o_mx  = o_fl + align256(fl);
+    const size_t    total = o_mx + align256(sizeof(double) * 2 * (size_t)c);
     if(h->size_query)
         return h->set_optimal_size(total);
     if((st = device_ready(h)) != rocblas_status_success)
@@ -2051,12 +2030,6 @@ rocblas_status trsm_refined_impl(rocblas_handle h, rocblas_side side, rocblas_fi
         return rocblas_status_internal_error;
     int*           err = ensure_err(h);
     unsigned char* ws  = reinterpret_cast<unsigned char*>(h->borrow(total));
-    if(!ws && plan.recursive)
-    {
-        plan = mixed_plan(pr, S, moduli, 64);
-        lay_out();
-        ws = reinterpret_cast<unsigned char*>(h->borrow(total));
-    }
     if(!ws || !err)
         return rocblas_status_memory_error;
     pr.err_dev = ps.err_dev = err;
@@ -2303,15 +2276,10 @@ rocblas_status trsm_mixed_host_impl(rocblas_handle h, rocblas_side side, rocblas
     const size_t inv_bytes = align256((size_t)kInvNB * k * sizeof(double));
     const size_t sl_bytes  = update_workspace_bytes(std::min(k, DB * kInvNB), n, k, slices, moduli,
                                                     pr.sm_count);
-    int          chain_w   = mixed_chain_width(pr);
+    const size_t ch_bytes  = mixed_chain_workspace_bytes(pr);
     const size_t ch_off    = inv_bytes + align256(sl_bytes);
     int*         err       = ensure_err(h);
-    void*        ws        = h->borrow(ch_off + align256(mixed_chain_workspace_bytes(pr, chain_w)));
-    if(!ws)
-    {
-        chain_w = 64; // its flags take least
-        ws      = h->borrow(ch_off + align256(mixed_chain_workspace_bytes(pr, chain_w)));
-    }
+    void*        ws        = h->borrow(ch_off + align256(ch_bytes));
     if(!ws || !err)
         return rocblas_status_memory_error;
     pr.err_dev = err;
@@ -2325,8 +2293,8 @@ rocblas_status trsm_mixed_host_impl(rocblas_handle h, rocblas_side side, rocblas
     rec.moduli   = moduli;
     rec.slice_ws = reinterpret_cast<unsigned char*>(ws) + inv_bytes;
     rec.err_dev  = err;
-    rec.chain_w  = chain_w;
-    if(mixed_chain_workspace_bytes(pr, chain_w))
+    rec.chain_w  = mixed_chain_width(pr);
+    if(ch_bytes)
         rec.chain_ws = reinterpret_cast<unsigned char*>(ws) + ch_off;
     for(int q = 0; q < nstep && rec.ok; ++q)
     {

@@ -573,8 +573,7 @@ static bool sliced_trsm_update(const TrsmProblem<T>& q, int c_lo, int c_hi, int 
     return run_sliced_gemm(g, ws, err, q.stream);
 }
 
-// Strip width of the precision form's chain sub-solves: that of the largest one on a whole device
-// (the width sizes the workspace, so it must not depend on the SMs that one call leaves to it).
+// Strip width of the precision form's chain sub-solves: that of the largest one on a whole device.
 static int mixed_chain_width(const TrsmProblem<double>& pr)
 {
     const int k = std::min<int64_t>((int64_t)tuning().mixed_chain_blocks * kInvNB, pr.k());
@@ -649,13 +648,13 @@ struct MixedRecursive : Recursive<double>
 };
 
 // Flags of the largest chain sub-solve of the precision form (0: no chain sub-solves).
-static size_t mixed_chain_workspace_bytes(const TrsmProblem<double>& pr, int w)
+static size_t mixed_chain_workspace_bytes(const TrsmProblem<double>& pr)
 {
     const int nbmax = tuning().mixed_chain_blocks;
     if(nbmax < 2)
         return 0;
     const int k = std::min<int64_t>((int64_t)nbmax * kInvNB, pr.k());
-    return chain_workspace_bytes(chain_shape(k, pr.side_left ? pr.n : pr.m, pr.batch, w));
+    return chain_workspace_bytes(chain_shape(k, pr.side_left ? pr.n : pr.m, pr.batch, 64));
 }
 
 // Largest sliced update of the recursion (the top node's off-diagonal block).

@@ -16,12 +16,13 @@
 //   * an item computes T = alpha C_b - sum over the finished blocks i of M_{b,i} X_i on DMMA
 //     (mma.sync m16n8k8 f64) from a ring of K chunks in shared memory, then X_b = inv(M_bb) T
 //     (the caller's or the fused trtri's invA block, its triangle masked), written over C_b, and
-//     releases the item's flag (CTA barrier, then st.release.gpu by one thread).
+//     advances the strip's count of finished blocks (CTA barrier, then st.release.gpu by one
+//     thread; blocks of a strip finish in order, so one count per strip is all that is waited on).
 //
 // The CTA is warp-specialised, because the FP64 tensor pipe (64 FMAs per clock and SM) is what
 // the work is bound by and every instruction that the MMA warps spend on copies is time it
 // idles: 8 warps only read fragments and issue MMAs, 3 warps copy M (and, after an item's last
-// chunk of M, its inverse block) and one warp waits for the flags of the finished blocks
+// chunk of M, its inverse block) and one warp waits for the strip's count
 // (ld.acquire.gpu) and copies X, each through cp.async whose completion arrives on the ring
 // slot's barrier.  The copies of M need no flag, so while the CTA waits for the block before its
 // own (the dependency chain, which is what few right-hand sides are bound by) that block's
@@ -108,7 +109,10 @@ struct ChainParams
     Scalar<T>      alpha;   // the caller's alpha
     int            conj = 0; // complex: M's entries are conjugated
     int            first;   // 1: this solve applies alpha; 0: it applies 1 (a sub-solve after an update)
-    int*           flags;   // one per item id, zero at launch
+    // finished blocks per (system, strip), zero at launch: blocks of a strip finish in solve order,
+    // so a count serves all their waits; one byte each where flag1 (then at most 255 blocks)
+    int*           flags;
+    int            flag1 = 0;
     int*           counter; // 8-byte claim counter, zero at launch
     int*           error;   // set to 4 if a wait timed out
     long long      wait_cycles = 1ll << 31; // a flag wait gives up after this many clock cycles
@@ -124,6 +128,18 @@ __device__ __forceinline__ int chain_ld_acquire(const int* p)
 __device__ __forceinline__ void chain_st_release(int* p, int v)
 {
     asm volatile("st.global.release.gpu.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ int chain_ld_acquire1(const void* p)
+{
+    int v;
+    asm volatile("ld.global.acquire.gpu.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void chain_st_release1(void* p, int v)
+{
+    asm volatile("st.global.release.gpu.u8 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 template <typename T>
@@ -208,8 +224,9 @@ struct ChainItem
     T*       C;     // C(0, c0) in B's storage
     int64_t  lda, ldb;
     int64_t  item;  // < 0: no more items
-    int*     flag0; // flag of solve position jj: flag0 + (VB ? vL[jj] : jj * fstride)
-    int64_t  fstride;
+    int*     flag0; // VB: flag of solve position jj is flag0[vL[jj]]; else the strip's count is
+    int64_t  fcell; // flags[fcell]
+    int      pos;   // solve position
     int      r0, bs, wv, nb, forward;
     int      klo, khi, ktop; // rows of the finished blocks [klo, khi), chunks counted from ktop when backward
     int      nk, nki;        // chunks of M and of the inverse
@@ -335,7 +352,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
             A = v.A; q.inv = v.invA; B = v.B; q.lda = v.lda; q.ldb = v.ldb;
             k = v.k; ncols = v.ncols; q.nb = v.nb; q.forward = v.forward;
             q.flag0   = H.flags + H.vP[a] + strip;
-            q.fstride = 0;
+            q.fcell   = 0;
         }
         else
         {
@@ -348,11 +365,12 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
             B     = reinterpret_cast<T*>(p.B.get(sysi));
             q.lda = p.lda * PT; q.ldb = p.ldb * PT; k = p.k * PT; ncols = p.ncols; q.nb = p.nb;
             q.forward = p.forward;
-            q.flag0   = p.flags + (int64_t)sysi * p.ns + strip;
-            q.fstride = (int64_t)p.systems * p.ns;
+            q.flag0   = nullptr;
+            q.fcell   = (int64_t)sysi * p.ns + strip;
         }
         const int b = q.forward ? j : q.nb - 1 - j;
         q.item = item;
+        q.pos  = j;
         q.r0   = b * kChainNB;
         q.bs   = min(kChainNB, k - q.r0);
         q.wv   = min(W, ncols - strip * W);
@@ -526,10 +544,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                 auto line_of = [&](int l) -> int64_t { return KCQ || !CX ? l * q.ldb : (l >> 1) * q.ldb + (l & 1); };
                 constexpr int kFastStep = KCQ ? 32 : 32 * PT;
                 constexpr uint32_t kDstLine = (uint32_t)sizeof(T) * kStep * Cfg::kPitchQ;
-                // solve positions [0, done) of the item's nprev earlier ones are known finished; one
-                // round of loads looks at the next 32 flags, so finished blocks cost no round trip each
-                const int nprev = q.forward ? q.r0 / kChainNB : q.nb - 1 - q.r0 / kChainNB;
-                int       done  = 0;
+                // solve positions [0, done) of the q.pos earlier ones are known finished; one round of
+                // loads learns of all that are (VB: of the next 32), so finished blocks cost no round
+                // trip each
+                int done = 0;
                 for(int i = 0; i < q.nk; ++i)
                 {
                     const int k0  = q.forward ? i * BK : q.ktop - (i + 1) * BK;
@@ -540,17 +558,19 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                         const long long t0 = clock64();
                         for(;;)
                         {
-                            const int jj = done + lane;
-                            int       f  = 0;
-                            if(jj < nprev)
+                            if constexpr(VB)
                             {
-                                if constexpr(VB)
-                                    f = chain_ld_acquire(q.flag0 + p.vhdr->vL[jj]);
-                                else
-                                    f = chain_ld_acquire(q.flag0 + jj * q.fstride);
+                                const int      jj    = done + lane;
+                                const int      f     = jj < q.pos ? chain_ld_acquire(q.flag0 + p.vhdr->vL[jj]) : 0;
+                                const unsigned ready = __ballot_sync(0xffffffffu, f != 0);
+                                done += ready == 0xffffffffu ? 32 : __ffs(~ready) - 1;
                             }
-                            const unsigned ready = __ballot_sync(0xffffffffu, f != 0);
-                            done += ready == 0xffffffffu ? 32 : __ffs(~ready) - 1;
+                            else
+                            {
+                                done = p.flag1 ? chain_ld_acquire1(reinterpret_cast<const char*>(p.flags) + q.fcell)
+                                               : chain_ld_acquire(p.flags + q.fcell);
+                                done = __reduce_min_sync(0xffffffffu, done); // (lanes load the same count)
+                            }
                             if(pos < done || __any_sync(0xffffffffu, aborted()))
                                 break;
                             if(__any_sync(0xffffffffu, clock64() - t0 > p.wait_cycles))
@@ -852,17 +872,28 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
         if(mma_sync_stop())
             break;
         if(tid == 0)
-            chain_st_release((VB ? p.vhdr->flags : p.flags) + q.item, 1);
+        {
+            if constexpr(VB)
+                chain_st_release(p.vhdr->flags + q.item, 1);
+            else if(p.flag1)
+                chain_st_release1(reinterpret_cast<char*>(p.flags) + q.fcell, q.pos + 1);
+            else
+                chain_st_release(p.flags + q.fcell, q.pos + 1);
+        }
         item_done(n);
     }
 }
 
-// Blocks, strips and the workspace of one uniform chain solve: flags (one per item), then
-// (8-byte aligned) the 8-byte claim counter and a spare error word.
+// Blocks, strips and the workspace of one uniform chain solve: the strips' counts, then (8-byte
+// aligned) the 8-byte claim counter and a spare error word.  The counts take one word per 128-row
+// block and 64-column strip, whatever the width: as words where that is enough for the strips, else
+// (narrow strips of a few blocks) as bytes.
 struct ChainShape
 {
     int     nb, ns, w;
     int64_t items;
+    int64_t words;  // of the counts' space
+    int     flag1;  // counts are bytes
 };
 
 inline ChainShape chain_shape(int k, int ncols, int batch, int w)
@@ -872,17 +903,16 @@ inline ChainShape chain_shape(int k, int ncols, int batch, int w)
     c.nb    = (int)ceil_div(k, kChainNB);
     c.ns    = (int)ceil_div(ncols, w);
     c.items = (int64_t)batch * c.nb * c.ns;
+    c.words = (int64_t)batch * c.nb * ceil_div(ncols, 64);
+    c.flag1 = (int64_t)batch * c.ns > c.words; // then nb < 8, and the counts fit as bytes
+    if(c.flag1 && (int64_t)batch * c.ns > 4 * c.words)
+        return chain_shape(k, ncols, batch, 64); // (one block of 8-column strips)
     return c;
-}
-
-inline size_t chain_flags_bytes(int64_t items)
-{
-    return ((size_t)items * sizeof(int) + 7) / 8 * 8 + 16;
 }
 
 inline size_t chain_workspace_bytes(const ChainShape& c)
 {
-    return chain_flags_bytes(c.items);
+    return ((size_t)c.words * sizeof(int) + 7) / 8 * 8 + 16;
 }
 
 // cluster2: the grid as clusters of two CTAs (placement only; the kernel uses no cluster

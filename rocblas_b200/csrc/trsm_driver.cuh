@@ -505,6 +505,7 @@ static void launch_chain_sub(const TrsmProblem<T>& pr, int b0, int b1, int first
     const int        kk    = std::min(b1 * NB, pr.k()) - r0;
     const int        ncols = pr.side_left ? pr.n : pr.m;
     const ChainShape cs    = chain_shape(kk * PT, ncols, pr.batch, w);
+    w                      = cs.w;
     int*             flags = reinterpret_cast<int*>(ws);
     cudaMemsetAsync(flags, 0, chain_workspace_bytes(cs), pr.stream);
     ChainParams<T> c{};
@@ -524,8 +525,9 @@ static void launch_chain_sub(const TrsmProblem<T>& pr, int b0, int b1, int first
     c.alpha   = pr.alpha;
     c.first   = first;
     c.flags   = flags;
+    c.flag1   = cs.flag1;
     // the 8-byte claim counter and the error word follow the flags
-    const size_t tail = ((size_t)cs.items * sizeof(int) + 7) / 8 * 8;
+    const size_t tail = ((size_t)cs.words * sizeof(int) + 7) / 8 * 8;
     c.counter = reinterpret_cast<int*>(reinterpret_cast<char*>(flags) + tail);
     // the error word: the handle's, else a slot after the counter
     c.error       = pr.err_dev ? pr.err_dev : c.counter + 2;

@@ -1,6 +1,6 @@
 """The chain solve (trsm_chain.cuh) at every strip width and at ragged strips, blocks and leading
-dimensions, forward and backward, both element types; a workspace that holds only the widest
-strips' flags is still used; and the inverse-block kernel (trtri_block.cuh) at its tile edges."""
+dimensions, forward and backward, both element types; the workspace does
+not depend on the width; and the inverse-block kernel (trtri_block.cuh) at its tile edges."""
 import ctypes
 import itertools
 
@@ -48,10 +48,10 @@ def test_widths(width, w, dtype):
         assert rb.lib().rocblas_b200_get_device_error(h.value, ctypes.byref(code)) == 0 and code.value == 0
 
 
-def test_workspace_of_the_widest_strips(width):
-    """A fixed workspace too small for the flags of narrow strips, but large enough for those of
-    the widest: the blocked solve runs, not the degraded one."""
-    k, cols = 1000, 48
+@pytest.mark.parametrize("k,cols", [(1000, 48), (200, 300), (140, 8)])
+def test_workspace_does_not_depend_on_the_width(width, k, cols):
+    """The strips' counts share the space of one word per block and 64-column strip, as words or
+    (few blocks, narrow strips) as bytes; a fixed workspace of the queried size is enough."""
     L = rb.lib()
 
     def query(h, w):
@@ -63,14 +63,16 @@ def test_workspace_of_the_widest_strips(width):
         assert L.rocblas_stop_device_memory_size_query(h.value, ctypes.byref(size)) == 0
         return size.value
 
+    A, B = oracle.nan_triangle_problem(5, "L", "L", "N", "N", k, cols, k, k, np.float64)
+    X = oracle.trsm("L", "L", "N", "N", 1.25, A, B)
     with rb.Handle() as h:
-        wide = query(h, 64)
-        assert query(h, 8) > wide
-        assert L.rocblas_set_device_memory_size(h.value, wide) == 0
-        A, B = oracle.nan_triangle_problem(5, "L", "L", "N", "N", k, cols, k, k, np.float64)
-        out = _solve(h, "L", "L", "N", "N", k, cols, A, B)  # status success, not perf_degraded
-        X = oracle.trsm("L", "L", "N", "N", 1.25, A, B)
-        assert oracle.matrix_norm_1(X, out) <= oracle.trsm_tolerance(np.float64, k)
+        sizes = [query(h, w) for w in (8, 16, 32, 64)]
+        assert len(set(sizes)) == 1
+        assert L.rocblas_set_device_memory_size(h.value, sizes[0]) == 0
+        for w in (8, 16, 32, 64):
+            assert width(w) == 0
+            out = _solve(h, "L", "L", "N", "N", k, cols, A, B)
+            assert oracle.matrix_norm_1(X, out) <= oracle.trsm_tolerance(np.float64, k)
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
