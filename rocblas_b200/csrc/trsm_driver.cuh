@@ -325,9 +325,10 @@ struct Recursive
     }
 };
 
-// Build invA for all diagonal blocks of A (k x k) into `inv` (ld 128, stride 128*128).
+// Build invA for all diagonal blocks of A (k x k) into `inv` (ld 128, stride 128*128); `alpha` as in
+// TrtriParams.
 template <typename T>
-static void build_invA(const TrsmProblem<T>& pr, BatchPtr<T> inv)
+static void build_invA(const TrsmProblem<T>& pr, BatchPtr<T> inv, const Scalar<T>& alpha = Scalar<T>{})
 {
     const int      k = pr.k();
     TrtriParams<T> t{};
@@ -340,11 +341,13 @@ static void build_invA(const TrsmProblem<T>& pr, BatchPtr<T> inv)
     t.inv_block_stride = (int64_t)kInvNB * kInvNB;
     t.upper = pr.upper;
     t.unit = pr.unit;
+    t.alpha = alpha;
     launch_trtri<T>(t, (int)ceil_div(k, kInvNB), pr.batch, pr.stream);
 }
 
 // Inverses of a complex A's diagonal blocks of kCplxNB rows (ld kCplxNB), for the chain: the block
-// solver on identities, all blocks in one launch.
+// solver on identities, all blocks in one launch.  (These are sub-solves that apply 1; with the
+// caller's alpha 0 they read nothing of A, as the chain then reads nothing of them.)
 constexpr int kCplxNB = kInvNB / 2;
 
 template <typename T>
@@ -365,19 +368,18 @@ static void build_cplx_inverses(const TrsmProblem<T>& pr, BatchPtr<T> inv)
     TrsmProblem<T> q = pr;
     q.side_left = 1;
     q.trans = q.conj = 0;
-    q.alpha = Scalar<T>{};
     q.ldb   = kCplxNB;
     q.batch = k / kCplxNB;
     BatchPtr<T> A = pr.A, X = inv;
     A.stride = (int64_t)kCplxNB * (pr.lda + 1);
     X.stride = (int64_t)kCplxNB * kCplxNB;
     if(q.batch)
-        launch_block_solve<T>(q, kCplxNB, kCplxNB, A, X, 1);
+        launch_block_solve<T>(q, kCplxNB, kCplxNB, A, X, 0);
     if(const int rem = k % kCplxNB)
     {
         const int64_t b = q.batch;
         q.batch = 1;
-        launch_block_solve<T>(q, rem, rem, A.shifted(b * A.stride), X.shifted(b * X.stride), 1);
+        launch_block_solve<T>(q, rem, rem, A.shifted(b * A.stride), X.shifted(b * X.stride), 0);
     }
 }
 
@@ -622,7 +624,7 @@ static void trsm_run(TrsmProblem<T> pr, void* ws, bool supplied_invA)
                 BatchPtr<T> inv;
                 inv.base   = reinterpret_cast<T*>(ws);
                 inv.stride = (int64_t)kInvNB * k;
-                build_invA<T>(pr, inv);
+                build_invA<T>(pr, inv, pr.alpha);
                 pr.invA = inv;
             }
             else

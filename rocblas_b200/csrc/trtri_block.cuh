@@ -46,6 +46,9 @@ struct TrtriParams
     // pointer arrays); blocks beyond an entry's order exit at once
     const int*     vk   = nullptr;
     const int64_t* vlda = nullptr;
+    // the alpha of the solve that the inverses are for: with 0 it reads neither them nor A, which
+    // need not exist then, so nothing is done
+    Scalar<T> alpha;
 };
 
 constexpr int kTrtriNB      = 128;
@@ -163,6 +166,8 @@ __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<
     double* Tm = X + kTrtriNB * kTrtriLd;
 
     const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if(p.alpha.get() == T(0))
+        return;
     const int     blk   = blockIdx.x;
     const int     batch = p.batch_base + blockIdx.y;
     const int     k     = p.vk ? p.vk[batch] : p.k;
