@@ -5,6 +5,11 @@
 namespace rb200
 {
 
+__device__ __forceinline__ bool is_finite(double v)
+{
+    return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
+}
+
 // mma.sync m16n8k8 .f64 (sm_90+ shape; 1024 FMAs per instruction).  Fragments, with
 // g = lane / 4 and t = lane % 4: A (16x8): a0 (g, t), a1 (g+8, t), a2 (g, t+4), a3 (g+8, t+4);
 // B (8x8): b0 (t, g), b1 (t+4, g); C (16x8): c0 (g, 2t), c1 (g, 2t+1), c2 (g+8, 2t), c3 (g+8, 2t+1).

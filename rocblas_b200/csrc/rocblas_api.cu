@@ -272,8 +272,11 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
         }
     }
 
+    // solved by substitution where it is not the chain's: orders of the strip solver, complex systems
+    const bool substitutes = is_cplx<T>::value || choose_algo(pr) == Algo::block;
     pr.chain_small = 1;
     pr.chain_small = use_chain(pr);
+    pr.subst       = pr.chain_small && substitutes;
     const size_t ws_bytes = trsm_workspace_bytes<T>(pr, have_invA);
     if(h->size_query)
         return ws_bytes ? h->set_optimal_size(ws_bytes) : rocblas_status_size_unchanged;
@@ -294,9 +297,7 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
         {
             // a workspace too small for this path: the strip solver, where it can take the order,
             // and the complex recursion need none, the recursive FP32 solve no counts
-            TrsmProblem<T> small = pr;
-            small.chain_small    = 0;
-            if(is_cplx<T>::value || choose_algo(small) == Algo::block)
+            if(substitutes)
             {
                 pr.chain_small = 0;
                 pr.chain_w     = is_cplx<T>::value ? -1 : 0;

@@ -111,11 +111,6 @@ __device__ __forceinline__ void ss_pair(const float* tile, int pair, double& b0,
     b1 = (double)v.y;
 }
 
-__device__ __forceinline__ bool ss_finite(double v)
-{
-    return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
-}
-
 // One strip: columns s0 .. s0 + 31 (of ncols) of C.  NS: panels in the ring.
 template <typename T, int RT, int NS>
 __device__ __forceinline__ void strip_solve(const T* A, int64_t lda, T* B, int64_t ldb, int k, int side_left, int tM,
@@ -336,7 +331,7 @@ __device__ __forceinline__ void strip_solve(const T* A, int64_t lda, T* B, int64
 #pragma unroll
                 for(int i = 0; i < 8; ++i)
                 {
-                    fin = fin && ss_finite(s[i]);
+                    fin = fin && is_finite(s[i]);
                     inv[q * 64 + ss_elem<double>(i, c)] = s[i];
                 }
                 bad = __ballot_sync(0xffffffffu, !fin);
@@ -349,7 +344,7 @@ __device__ __forceinline__ void strip_solve(const T* A, int64_t lda, T* B, int64
                 double       x[2] = {0.0, 0.0};
                 const double T0 = cv[Q][0] - acc[s][0], T1 = cv[Q][1] - acc[s][1];
                 const bool plain = ((bad >> (8 * Q)) & 0xff) == 0
-                                   && __all_sync(0xffffffffu, ss_finite(T0) && ss_finite(T1));
+                                   && __all_sync(0xffffffffu, is_finite(T0) && is_finite(T1));
                 if(plain)
                 {
                     double b0, b1;

@@ -48,6 +48,14 @@
 // M(r, c) = tM ? A(c, r) : A(r, c).  Blocks are solved in increasing order when M is lower
 // and in decreasing order when M is upper; the K chunks of an item follow the same order.
 // Unit diagonals need nothing here: invA already holds the inverse of the unit triangle.
+//
+// A product with an inverse is not a substitution where something is not finite: the zeros beside
+// the triangle turn an infinity of T into NaNs in rows that do not depend on it, and the real
+// inverses read a zero diagonal entry as 1.  Systems that a substituting solver would take
+// otherwise (ChainParams::subst) must answer as that solver does, so an item of theirs whose X is
+// not finite, or whose block has a zero on its diagonal, is solved again from T by substitution
+// (chain_substitute).  X finite means that nothing else was in the product: an entry of T or of
+// the triangle that is not finite makes the entry of X in its own row so.
 #pragma once
 #include "gemm_dmma.cuh"
 #include "mbarrier.cuh"
@@ -108,6 +116,9 @@ struct ChainParams
     const ChainVbHeader<T>* vhdr;
     Scalar<T>      alpha;   // the caller's alpha
     int            conj = 0; // complex: M's entries are conjugated
+    int            unit = 0; // as in BlockSolveParams; only read by a SUBST kernel
+    int            subst = 0; // infinities, NaNs and zero diagonals as in a substitution (real types;
+                              // complex ones always)
     int            first;   // 1: this solve applies alpha; 0: it applies 1 (a sub-solve after an update)
     // finished blocks per (system, strip), zero at launch: blocks of a strip finish in solve order,
     // so a count serves all their waits; one byte each where flag1 (then at most 255 blocks)
@@ -232,9 +243,81 @@ struct ChainItem
     int      nk, nki;        // chunks of M and of the inverse
 };
 
+// C(r0 + o, col) of an item
+template <typename T, int PT, bool KCQ>
+__device__ __forceinline__ T* chain_caddr(const ChainItem<T>& q, int o, int col)
+{
+    const int r = q.r0 + o;
+    return KCQ       ? q.C + r + (int64_t)col * q.ldb
+           : PT == 2 ? q.C + 2 * col + (int64_t)(r >> 1) * q.ldb + (r & 1)
+                     : q.C + col + (int64_t)r * q.ldb;
+}
+
+// An item's block by substitution from T (Ts, [row][column] with the given pitch), in place and over
+// C_b, by the MMA warps.  The reciprocal of the diagonal is multiplied, as the substituting solvers do.
+template <typename TT, int W, bool KCP, bool KCQ>
+__device__ __noinline__ void chain_substitute(double* Ts, int pitch, const ChainItem<typename ChainReal<TT>::type>& q,
+                                              int unit, int conj)
+{
+    using T = typename ChainReal<TT>::type;
+    constexpr int PT = ChainReal<TT>::parts, G = kChainMmaThreads / W;
+    const int     rows = q.bs / PT, col = threadIdx.x % W, grp = threadIdx.x / W;
+    auto entry = [&](int i, int j, double& re, double& im) {
+        const auto* e = KCP ? q.M + i * q.lda + q.r0 + PT * j : q.M + PT * i + (q.r0 / PT + j) * q.lda;
+        re = (double)e[0];
+        if constexpr(PT == 2)
+            im = conj ? -(double)e[1] : (double)e[1];
+    };
+    // rows solved one after another; a row's value reaches Ts once nobody reads it for an update
+    for(int s = 0; s < rows; ++s)
+    {
+        const int j = q.forward ? s : rows - 1 - s;
+        double    dr = 1.0, di = 0.0;
+        if(unit != 1)
+            entry(j, j, dr, di);
+        if(unit == 2 && dr == 0.0 && di == 0.0)
+            dr = 1.0;
+        double* const row = Ts + PT * j * pitch + col;
+        double        xr = row[0], xi = 0.0;
+        if constexpr(PT == 2)
+        {
+            const cplx<double> x = cplx<double>(xr, row[pitch]) * (cplx<double>(1.0) / cplx<double>(dr, di));
+            xr = x.x;
+            xi = x.y;
+        }
+        else
+            xr *= 1.0 / dr;
+        for(int d = 1 + grp; d < rows - s; d += G)
+        {
+            const int i = q.forward ? j + d : j - d;
+            double    mr, mi = 0.0;
+            entry(i, j, mr, mi);
+            double* const c = Ts + PT * i * pitch + col;
+            if constexpr(PT == 2)
+            {
+                c[0] -= mr * xr - mi * xi;
+                c[pitch] -= mr * xi + mi * xr;
+            }
+            else
+                c[0] -= mr * xr;
+        }
+        asm volatile("barrier.cta.sync 1, %0;" ::"n"(kChainMmaThreads) : "memory");
+        if(grp == 0)
+        {
+            row[0] = xr;
+            if constexpr(PT == 2)
+                row[pitch] = xi;
+        }
+    }
+    asm volatile("barrier.cta.sync 1, %0;" ::"n"(kChainMmaThreads) : "memory");
+    for(int o = grp; o < q.bs && col < q.wv; o += G)
+        *chain_caddr<T, PT, KCQ>(q, o, col) = (T)Ts[o * pitch + col];
+}
+
 // W right-hand sides per item (8, 16, 32 or 64).  KCP: M's K index is contiguous in memory (tM);
 // KCQ: C's row index is contiguous (side L).  VB: the variable-size tables of p describe the items.
-template <typename TT, int W, bool KCP, bool KCQ, bool VB>
+// SUBST: ChainParams::subst; a kernel of its own, since the checks and the call cost the others 1 to 4%.
+template <typename TT, int W, bool KCP, bool KCQ, bool VB, bool SUBST>
 __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParams<TT> p)
 {
     using Cfg = ChainCfg<TT, W, KCP, KCQ>;
@@ -248,6 +331,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
     __shared__ ChainItem<T> s_item[2];
     __shared__ uint64_t     full[NS], empty[NS], item_full[2], item_empty[2];
     __shared__ int          s_abort;
+    __shared__ int          s_zero[2]; // SUBST: the item's block has a zero on its diagonal
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if(tid == 0)
@@ -386,15 +470,15 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
         q.nki  = zero ? 0 : (int)ceil_div(q.bs, BK);
     };
     // barrier of the MMA warps; true in all of them if any saw a wait run out, so that they leave
-    // the item loop together
-    auto mma_sync_stop = [&]() -> bool {
+    // the item loop together, or passed a reason of its own
+    auto mma_sync_stop = [&](bool why = false) -> bool {
         int any;
         asm volatile("{\n\t.reg .pred p, q;\n\t"
                      "setp.ne.s32 p, %1, 0;\n\t"
                      "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
                      "selp.s32 %0, 1, 0, q;\n\t}"
                      : "=r"(any)
-                     : "r"((int)aborted()), "n"(kChainMmaThreads)
+                     : "r"((int)(why || aborted())), "n"(kChainMmaThreads)
                      : "memory");
         return any != 0;
     };
@@ -548,6 +632,20 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                 // loads learns of all that are (VB: of the next 32), so finished blocks cost no round
                 // trip each
                 int done = 0;
+                // (SUBST) the block's diagonal; a complex zero needs no look, it makes the inverse NaN
+                constexpr bool kDiag = SUBST && !CX;
+                T              diag[kChainNB / 32];
+                if constexpr(kDiag)
+                {
+#pragma unroll
+                    for(int u = 0; u < kChainNB / 32; ++u)
+                    {
+                        const int o = lane + 32 * u;
+                        diag[u]     = T(1);
+                        if(!zero && !p.unit && o < q.bs)
+                            diag[u] = KCP ? q.M[o * q.lda + q.r0 + o] : q.M[o + (q.r0 + o) * q.lda];
+                    }
+                }
                 for(int i = 0; i < q.nk; ++i)
                 {
                     const int k0  = q.forward ? i * BK : q.ktop - (i + 1) * BK;
@@ -614,6 +712,17 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
                 for(int i = 0; i < q.nki; ++i)
                 {
                     slot();
+                    if(kDiag && i + 1 == q.nki)
+                    {
+                        bool z = false;
+#pragma unroll
+                        for(int u = 0; u < kChainNB / 32; ++u)
+                            z = z || diag[u] == T(0);
+                        z = __any_sync(0xffffffffu, z);
+                        if(lane == 0)
+                            s_zero[n & 1] = z; // read after the last chunk's barrier
+                        __syncwarp();
+                    }
                     mbar_arrive(&full[st]); // its share of the slot's arrivals
                     advance();
                 }
@@ -679,12 +788,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
         if(q.item < 0)
             break;
         // C(r0 + o, col) of this thread's output (i, jn, e)
-        auto caddr = [&](int o, int col) -> T* {
-            const int r = q.r0 + o;
-            return KCQ  ? q.C + r + (int64_t)col * q.ldb
-                   : CX ? q.C + 2 * col + (int64_t)(r >> 1) * q.ldb + (r & 1)
-                        : q.C + col + (int64_t)r * q.ldb;
-        };
+        auto caddr = [&](int o, int col) -> T* { return chain_caddr<T, PT, KCQ>(q, o, col); };
         auto out_o = [&](int i, int e) { return row0 + i * 16 + g + (e >> 1) * 8; };
         auto out_n = [&](int jn, int e) { return col0 + jn * 8 + 2 * t + (e & 1); };
 
@@ -853,6 +957,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
 
         // ---- 4. X_b over C_b, then release the item's flag ---------------------------------
         const bool live = !aborted();
+        bool       redo = false; // (SUBST) not what a substitution gives
+        if constexpr(SUBST && !CX)
+            redo = q.nki > 0 && s_zero[n & 1];
 #pragma unroll
         for(int i = 0; i < TM; ++i)
 #pragma unroll
@@ -865,12 +972,25 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
 #pragma unroll
                     for(int s = 1; s < SP; ++s)
                         v += acc[s][i][jn][e];
+                    if constexpr(SUBST)
+                        redo = redo || !is_finite(v); // (0 outside C_b unless something in it is not)
                     if(live && o < q.bs && col < q.wv)
                         *caddr(o, col) = (T)v;
                 }
         // all of X_b is written (and T free for the next item) once every MMA warp is here
-        if(mma_sync_stop())
-            break;
+        if constexpr(!SUBST)
+        {
+            if(mma_sync_stop())
+                break;
+        }
+        else if(mma_sync_stop(redo))
+        {
+            if(mma_sync_stop())
+                break;
+            chain_substitute<TT, W, KCP, KCQ>(Ts, Cfg::kPitchT, s_item[n & 1], p.unit, p.conj);
+            if(mma_sync_stop())
+                break;
+        }
         if(tid == 0)
         {
             if constexpr(VB)
@@ -922,7 +1042,10 @@ static void launch_chain_cfg(const ChainParams<T>& p, int sms, int64_t max_items
                              bool cluster2 = false)
 {
     using Cfg = ChainCfg<T, W, KCP, KCQ>;
-    auto kern = trsm_chain_kernel<T, W, KCP, KCQ, VB>;
+    auto kern = trsm_chain_kernel<T, W, KCP, KCQ, VB, is_cplx<T>::value>;
+    if constexpr(!is_cplx<T>::value && !VB)
+        if(p.subst)
+            kern = trsm_chain_kernel<T, W, KCP, KCQ, VB, true>;
     cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kChainThreads, Cfg::kSmem);

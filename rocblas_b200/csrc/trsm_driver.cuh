@@ -69,6 +69,7 @@ struct TrsmProblem
                                  // are whole SM pairs (set beside a kernel placed in pairs)
     int         chain_w = 0; // strip width of the chain solve (0: chain_width's choice; < 0: no chain)
     int         chain_small = 0; // orders the strip solver could take may go to the chain (choose_algo)
+    int         subst = 0; // the chain takes it from a solver that substitutes (ChainParams::subst)
     int         k() const { return side_left ? m : n; }
     // op(A) lower?
     int oplower() const { return (!upper) != (trans != 0); }
@@ -515,6 +516,8 @@ static void launch_chain_sub(const TrsmProblem<T>& pr, int b0, int b1, int first
     c.lda     = pr.lda;
     c.invA    = pr.invA.shifted((int64_t)b0 * NB * NB);
     c.conj    = pr.conj;
+    c.unit    = pr.unit;
+    c.subst   = pr.subst;
     c.B       = pr.B.shifted(pr.side_left ? (int64_t)r0 : (int64_t)r0 * pr.ldb);
     c.ldb     = pr.ldb;
     c.k       = kk;
