@@ -88,9 +88,13 @@ __device__ __forceinline__ void trtri_mma(double (&acc)[NT][4], const double* P,
 
 // The inverse of the lower triangular 128 x 128 block at X (column-major, pitch kTrtriLd, zero above
 // the diagonal), in place, by 256 threads between two CTA barriers (the caller's before it, the
-// last of its own after it).  Tm: 64 columns of kTrtriLdT doubles.
-__device__ __forceinline__ void trtri_invert(double* X, double* Tm, bool zero_is_one)
+// last of its own after it).  Tm: 64 columns of kTrtriLdT doubles.  Returns (in all threads) whether
+// everything it wrote is finite: if not, the zeros of a triangle may have met an infinity or NaN in a
+// product, and rows may not be finite that do not depend on it; the caller then stages the block again
+// for trtri_invert_rows.
+__device__ __forceinline__ bool trtri_invert(double* X, double* Tm, bool zero_is_one)
 {
+    bool finite = true;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     // ---- 16 x 16 diagonal tiles: warp w inverts tile w, lane = column ----------------------------
@@ -117,7 +121,10 @@ __device__ __forceinline__ void trtri_invert(double* X, double* Tm, bool zero_is
         if(lane < S)
 #pragma unroll
             for(int i = 0; i < S; ++i)
+            {
+                finite                 = finite && (i < lane || is_finite(x[i]));
                 D[lane * kTrtriLd + i] = x[i];
+            }
     }
     __syncthreads();
 
@@ -147,8 +154,12 @@ __device__ __forceinline__ void trtri_invert(double* X, double* Tm, bool zero_is
         for(int n = 0; n < NT; ++n)
 #pragma unroll
             for(int e = 0; e < 4; ++e)
+            {
+                finite = finite && is_finite(acc[n][e]);
                 L21[(cb + 8 * n + 2 * t + (e & 1)) * kTrtriLd + rb + g + (e >> 1) * 8] = -acc[n][e];
-        __syncthreads();
+            }
+        if(S < kTrtriNB / 2)
+            __syncthreads();
     };
     doubling(std::integral_constant<int, 16>{}, std::integral_constant<int, 1>{}, warp >> 1, 0, (warp & 1) * 8);
     doubling(std::integral_constant<int, 32>{}, std::integral_constant<int, 2>{}, warp >> 2, (warp & 1) * 16,
@@ -156,6 +167,33 @@ __device__ __forceinline__ void trtri_invert(double* X, double* Tm, bool zero_is
     // warps w and w + 4 share a scheduler: opposite row blocks give it even work in both products
     doubling(std::integral_constant<int, 64>{}, std::integral_constant<int, 4>{}, 0,
              (warp < 4 ? warp : 7 - warp) * 16, (warp >> 2) * 32);
+    return __syncthreads_and(finite) != 0;
+}
+
+// The same inverse with products over the triangles alone, so that what is not finite stays in the
+// rows from its own on, as in a substitution: column after column from the last one,
+// X21 = -X22 l21 / l11, thread = row.  About 0.1 ms.
+__device__ __noinline__ void trtri_invert_rows(double* X, bool zero_is_one)
+{
+    const int r = threadIdx.x;
+    for(int c = kTrtriNB - 1; c >= 0; --c)
+    {
+        const double* const l = X + c * kTrtriLd;
+        double              d = l[c], v = 0.0;
+        if(zero_is_one && d == 0.0)
+            d = 1.0;
+        const double rd = 1.0 / d;
+        if(r > c && r < kTrtriNB)
+        {
+            for(int k = c + 1; k <= r; ++k)
+                v += X[k * kTrtriLd + r] * l[k];
+            v = -v * rd;
+        }
+        __syncthreads();
+        if(r >= c && r < kTrtriNB)
+            X[c * kTrtriLd + r] = r == c ? rd : v;
+        __syncthreads();
+    }
 }
 
 template <typename T>
@@ -189,45 +227,52 @@ __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<
         take = i < bs && j < bs && (j < i || (i == j && !p.unit));
         return take ? A0 + sg * (i + (int64_t)j * lda) : A0;
     };
-    if constexpr(std::is_same<T, double>::value)
-    {
-#pragma unroll
-        for(int c = 0; c < kTrtriNB / 8; ++c)
-#pragma unroll
-            for(int u = c / 4; u < kTrtriNB / 32; ++u)
-            {
-                const int i = u * 32 + lane, j = c * 8 + warp;
-                bool      take;
-                const T*  src = source(i, j, take);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(X + j * kTrtriLd + i)),
-                             "l"(src), "r"(take ? 8 : 0)
-                             : "memory");
-            }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-    }
-    else
-    {
-        // converted on the way: a row group's loads are all issued before its stores
-#pragma unroll
-        for(int u = 0; u < kTrtriNB / 32; ++u)
+    auto stage = [&]() {
+        if constexpr(std::is_same<T, double>::value)
         {
-            T v[4 * (kTrtriNB / 32)];
 #pragma unroll
-            for(int c = 0; c < 4 * (u + 1); ++c)
-            {
-                bool     take;
-                const T* src = source(u * 32 + lane, c * 8 + warp, take);
-                v[c]         = take ? *src : T(0);
-            }
+            for(int c = 0; c < kTrtriNB / 8; ++c)
 #pragma unroll
-            for(int c = 0; c < 4 * (u + 1); ++c)
-                X[(c * 8 + warp) * kTrtriLd + u * 32 + lane] = (double)v[c];
+                for(int u = c / 4; u < kTrtriNB / 32; ++u)
+                {
+                    const int i = u * 32 + lane, j = c * 8 + warp;
+                    bool      take;
+                    const T*  src = source(i, j, take);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(X + j * kTrtriLd + i)),
+                                 "l"(src), "r"(take ? 8 : 0)
+                                 : "memory");
+                }
+            asm volatile("cp.async.wait_all;" ::: "memory");
         }
-    }
-    __syncthreads();
+        else
+        {
+            // converted on the way: a row group's loads are all issued before its stores
+#pragma unroll
+            for(int u = 0; u < kTrtriNB / 32; ++u)
+            {
+                T v[4 * (kTrtriNB / 32)];
+#pragma unroll
+                for(int c = 0; c < 4 * (u + 1); ++c)
+                {
+                    bool     take;
+                    const T* src = source(u * 32 + lane, c * 8 + warp, take);
+                    v[c]         = take ? *src : T(0);
+                }
+#pragma unroll
+                for(int c = 0; c < 4 * (u + 1); ++c)
+                    X[(c * 8 + warp) * kTrtriLd + u * 32 + lane] = (double)v[c];
+            }
+        }
+        __syncthreads();
+    };
+    stage();
 
     // unit diagonals and padding are staged as 0, which like a zero diagonal entry is read as 1
-    trtri_invert(X, Tm, true);
+    if(!trtri_invert(X, Tm, true))
+    {
+        stage();
+        trtri_invert_rows(X, true);
+    }
 
     // ---- write inv(A_block) (bs x bs, ld = ldinv), zeros in the opposite triangle ----
     T* const out0 = p.upper ? out + (int64_t)(bs - 1) * (p.ldinv + 1) : out;

@@ -198,3 +198,28 @@ def test_rounding_error(width, uplo, w, dtype):
     d = dm.to_host(dB) - X
     error = np.sqrt((abs(d) ** 2).sum() / (abs(X) ** 2).sum())
     assert error <= (0.8 if dtype == np.float64 else 0.95) * 2.0**-53, error / 2.0**-53
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("i,j", [(5, 2), (20, 3), (27, 17), (50, 3), (120, 60), (127, 0)])
+def test_inverse_block_of_a_non_finite_entry(i, j, bad, dtype):
+    """Rows of the inverse before the entry's do not depend on it, nor do the columns after its own;
+    a substitution leaves them finite."""
+    n = 128
+    rng = np.random.default_rng(i)
+    T = np.tril(rng.uniform(-1, 1, (n, n)) / n, -1) + np.diag(rng.uniform(1, 2, n))
+    T[i, j] = bad
+    with rb.Handle() as h:
+        for uplo in "LU":
+            M = T if uplo == "L" else T[::-1, ::-1]
+            dA = dm.to_device(np.asfortranarray(M, dtype=dtype))
+            dX = dm.empty(n, n, dA.dtype, fill=0.0)
+            dm.trtri(h, uplo, "N", n, dA, n, dX, n)
+            torch.cuda.synchronize()
+            X = dm.to_host(dX)
+            X = X if uplo == "L" else X[::-1, ::-1]
+            assert np.isfinite(X[:i]).all() and np.isfinite(X[:, j + 1:]).all()
+            assert not np.isfinite(X[i, j]) and (np.triu(X, 1) == 0).all()
+            Y = np.linalg.inv(T[:i, :i].astype(dtype).astype(np.float64))
+            assert np.abs(X[:i, :i] - Y).max() <= 4 * n * np.finfo(dtype).eps

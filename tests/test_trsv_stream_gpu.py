@@ -74,3 +74,34 @@ def test_non_finite_entry_reaches_only_its_own_and_later_rows():
     with rb.Handle() as h:
         out = _trsv(h, np.float64, "L", "N", "N", n, A, n, b, 1)
     assert np.isfinite(out[:row]).all() and not np.isfinite(out[row:]).any()
+
+
+@pytest.mark.parametrize("trans", "NT")
+@pytest.mark.parametrize("what", ["nan", "inf", "zero", "overflow"])
+@pytest.mark.parametrize("pos,before", [(20, 3), (50, 20), (300, 260), (383, 256), (500, 30)])
+def test_rows_solved_before_a_bad_entry_of_a_stay_finite(pos, before, what, trans):
+    """An infinity, a NaN or a zero pivot of A reaches the row that holds it and those solved after it
+    (position = row for a lower triangle, from the end for its transpose); a pivot whose inverse row
+    overflows leaves the others finite."""
+    n = 700
+    A, B = oracle.nan_triangle_problem(9, "L", "L", trans, "N", n, 1, n, n, np.float64)
+    b = np.ascontiguousarray(B[:, 0])
+    order = np.arange(n) if trans == "N" else np.arange(n)[::-1]
+    r, c = order[pos], order[before]
+    M = A if trans == "N" else A.T
+    if what == "zero":
+        M[r, r] = 0
+    elif what == "overflow":
+        M[r, r], M[r, c] = 1e-300, 1e10
+    else:
+        M[r, c] = float(what)
+    with rb.Handle() as h:
+        out = _trsv(h, np.float64, "L", trans, "N", n, A, n, b, 1)[order]
+    assert np.isfinite(out[:pos]).all()
+    sub = order[:pos]
+    X = oracle.trsm("L", "L" if trans == "N" else "U", "N", "N", 1.0, np.asfortranarray(M[np.ix_(np.sort(sub), np.sort(sub))]),
+                    np.asfortranarray(b[np.sort(sub), None]))[:, 0]
+    X = X if trans == "N" else X[::-1]
+    assert np.abs(out[:pos] - X).max() <= oracle.trsm_tolerance(np.float64, n) * max(1.0, np.abs(X).max())
+    if what != "overflow":
+        assert not np.isfinite(out[pos:]).any()
