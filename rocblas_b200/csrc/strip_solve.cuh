@@ -26,9 +26,10 @@
 //     each lane reads back from where it wrote them in C;
 //   * a diagonal panel's four 8 x 8 tiles are inverted by each warp (lane = column, 28 FMAs) and
 //     every tile of the solve is then X = T inv^T, one more product, followed by the updates of
-//     the super-block's rows below.  Where a tile's inverse or right-hand side is not finite the
-//     tile is substituted row by row instead, so that an infinity or NaN reaches exactly the rows
-//     that it reaches in a substitution.
+//     the super-block's rows below.  Where that X is not finite (as it is where the inverse or the
+//     right-hand side is not, or where terms of the product overflow that a substitution would cancel
+//     before it divides) the tile is substituted row by row instead, so that an infinity or NaN
+//     reaches exactly the rows that it reaches in a substitution.
 // FP32 systems are staged as FP32 and computed in FP64.
 //
 // Measured (one B200, against the solver with the strip in shared memory and one-warp
@@ -307,7 +308,6 @@ __device__ __forceinline__ void strip_solve(const T* A, int64_t lda, T* B, int64
             if(!live)
                 return;
             // inverses of the four diagonal tiles: lane = (tile, column)
-            unsigned bad;
             {
                 const int q = lane >> 3, c = lane & 7;
                 const T*  D = S + ((P * 4 + q) * 4 + q) * 64;
@@ -326,15 +326,10 @@ __device__ __forceinline__ void strip_solve(const T* A, int64_t lda, T* B, int64
                     for(int i = j + 1; i < 8; ++i)
                         s[i] -= (double)D[ss_elem<T>(i, j)] * s[j];
                 }
-                bool fin = true;
                 __syncwarp(); // the previous panel's inverses are read
 #pragma unroll
                 for(int i = 0; i < 8; ++i)
-                {
-                    fin = fin && is_finite(s[i]);
                     inv[q * 64 + ss_elem<double>(i, c)] = s[i];
-                }
-                bad = __ballot_sync(0xffffffffu, !fin);
                 __syncwarp();
             }
             auto solve_tile = [&](auto q_const) {
@@ -343,16 +338,13 @@ __device__ __forceinline__ void strip_solve(const T* A, int64_t lda, T* B, int64
                     return;
                 double       x[2] = {0.0, 0.0};
                 const double T0 = cv[Q][0] - acc[s][0], T1 = cv[Q][1] - acc[s][1];
-                const bool plain = ((bad >> (8 * Q)) & 0xff) == 0
-                                   && __all_sync(0xffffffffu, is_finite(T0) && is_finite(T1));
-                if(plain)
                 {
                     double b0, b1;
                     ss_pair(inv + Q * 64 + pairD, 0, b0, b1);
                     dmma_8x8x4(x, T0, b0);
                     dmma_8x8x4(x, T1, b1);
                 }
-                else
+                if(!__all_sync(0xffffffffu, is_finite(x[0]) && is_finite(x[1])))
                 {
                     // row by row: the lane that holds row j scales it and hands it to its column's
                     // other lanes

@@ -88,3 +88,18 @@ def test_zero_diagonal(dtype):
     X = oracle.trsm("L", "L", "N", "N", 1.0, np.asfortranarray(A[:row, :row]), np.asfortranarray(B[:row]))
     assert oracle.matrix_norm_1(X, out[:row]) <= oracle.trsm_tolerance(dtype, k)
     assert np.isinf(out[row]).all() and not np.isfinite(out[row:]).any()
+
+
+@pytest.mark.parametrize("k", [2, 60, 100])
+def test_terms_that_overflow_and_cancel(k):
+    """The last row of [[1, 0], [1, 1e-300]] X = 1e10 has the solution 0; the product with the inverse
+    of the 2 x 2 block would subtract two infinities."""
+    A = np.asfortranarray(np.eye(k))
+    A[-1, -2], A[-1, -1] = 1, 1e-300
+    B = np.asfortranarray(np.full((k, 9), 1e10))
+    with rb.Handle() as h:
+        dA, dB = dm.to_device(A), dm.to_device(B)
+        dm.trsm(h, "L", "L", "N", "N", k, 9, 1.0, dA, k, dB, k)
+        torch.cuda.synchronize()
+    out = dm.to_host(dB)
+    assert (out[:-1] == 1e10).all() and (out[-1] == 0).all()
