@@ -292,11 +292,13 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
     void* ws = nullptr;
     if(ws_bytes)
     {
-        ws = h->borrow_optional(ws_bytes);
+        // a caller's buffer may start anywhere; these paths access it in units of up to 8 bytes
+        auto aligned = [](void* p) { return reinterpret_cast<uintptr_t>(p) % 8 ? nullptr : p; };
+        ws = aligned(h->borrow_optional(ws_bytes));
         if(!ws && use_chain(pr))
         {
             // a workspace too small for this path: the strip solver, where it can take the order,
-            // and the complex recursion need none, the recursive FP32 solve no counts
+            // and the complex recursion need none, the recursive FP32 solve no counts (and only floats)
             if(substitutes)
             {
                 pr.chain_small = 0;
@@ -307,10 +309,12 @@ rocblas_status trsm_impl(rocblas_handle h, rocblas_side side, rocblas_fill uplo,
                 if(std::is_same<T, float>::value && (pr.side_left ? pr.n : pr.m) > tuning().chain_max_cols_f32)
                     pr.chain_w = -1;
                 ws = h->borrow(trsm_workspace_bytes<T>(pr, have_invA));
+                if(pr.chain_w >= 0)
+                    ws = aligned(ws);
             }
         }
         else if(!ws)
-            ws = h->borrow(ws_bytes);
+            ws = aligned(h->borrow(ws_bytes));
         if(!ws && !have_invA && !is_cplx<T>::value && choose_algo(pr) != Algo::block)
         {
             // backup: recursive solve with block-solver leaves needs no workspace

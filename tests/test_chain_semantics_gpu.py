@@ -146,3 +146,18 @@ def test_supplied_inverse_blocks():
         torch.cuda.synchronize()
     out = dm.to_host(dB)
     assert np.isfinite(out[:r]).all() and np.isinf(out[r]).all() and not np.isfinite(out[r:]).any()
+
+
+@pytest.mark.parametrize("dtype,k,cols", SIZES + [(np.float32, 600, 700)])
+def test_workspace_that_starts_anywhere(dtype, k, cols):
+    """The caller's buffer has no alignment that the API asks for; what the chain cannot use goes to a
+    solver that can, with the same status."""
+    A, B, _ = _system("L", "L", "N", k, cols, dtype)
+    ws = torch.zeros(1 << 20, dtype=torch.float32, device="cuda")
+    with rb.Handle() as h:
+        assert rb.lib().rocblas_set_workspace(h.value, ctypes.c_void_p(ws.data_ptr() + 4), ws.numel() * 4 - 64) == 0
+        dA, dB = dm.to_device(A), dm.to_device(B)
+        dm.trsm(h, "L", "L", "N", "N", k, cols, 1.0, dA, k, dB, k)
+        torch.cuda.synchronize()
+    X = oracle.trsm("L", "L", "N", "N", 1.0, A, B)
+    assert oracle.matrix_norm_1(X, dm.to_host(dB)) <= oracle.trsm_tolerance(dtype, max(k, cols))
