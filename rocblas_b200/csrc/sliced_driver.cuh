@@ -573,11 +573,12 @@ static bool sliced_trsm_update(const TrsmProblem<T>& q, int c_lo, int c_hi, int 
     return run_sliced_gemm(g, ws, err, q.stream);
 }
 
-// Strip width of the precision form's chain sub-solves: that of the largest one on a whole device.
+// Strip width of the precision form's chain sub-solves: that of the largest one, for pr's SMs (the
+// callers pass the problem with the whole device's, also where a part of them solves it).
 static int mixed_chain_width(const TrsmProblem<double>& pr)
 {
     const int k = std::min<int64_t>((int64_t)tuning().mixed_chain_blocks * kInvNB, pr.k());
-    return chain_width(k, pr.side_left ? pr.n : pr.m, 1, 148);
+    return chain_width(k, pr.side_left ? pr.n : pr.m, 1, pr.sm_count);
 }
 
 // ---- precision form of the TRSM ---------------------------------------------------------------
