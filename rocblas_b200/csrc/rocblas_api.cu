@@ -641,6 +641,14 @@ rocblas_status trsv_impl(rocblas_handle h, rocblas_fill uplo, rocblas_operation 
                 p.flags = reinterpret_cast<int*>(ws);
                 p.error = err;
                 p.wait_cycles = 1ll << tuning().wait_cycles_log2;
+                if(stream && tuning().chain_first_item > 0)
+                {
+                    // failure injection (tests): the blocks before it are never claimed
+                    chain_set_counter_kernel<<<1, 1, 0, h->stream>>>(
+                        reinterpret_cast<int*>(reinterpret_cast<char*>(ws) + trsv_stream_exchange_bytes<T>(n)),
+                        tuning().chain_first_item);
+                    count_launch();
+                }
                 if(stream && p.trans)
                     launch_trsv_stream<T, true>(p, reinterpret_cast<T*>(ws), nblk, h->sm_count, h->stream);
                 else if(stream)

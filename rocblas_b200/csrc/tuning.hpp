@@ -62,9 +62,10 @@ struct Tuning
     int strsm_sliced_min_k   = 1024; // ... for updates with at least this inner dimension
     int mixed_moduli         = 16;   // precision form: 0 updates on the slice engine; 14..16 on
                                      // the residue (CRT) engine with this many moduli
-    int chain_first_item     = 0;    // failure injection for tests: uniform chain launches start
-                                     // claiming items here, so the flags of the items before it
-                                     // are never set and the waits on them run out (0: off)
+    int chain_first_item     = 0;    // failure injection for tests: uniform chain launches and the
+                                     // streaming TRSV start claiming items here, so the flags of
+                                     // the items before it are never set and the waits on them
+                                     // run out (0: off)
 };
 
 struct TuningEntry

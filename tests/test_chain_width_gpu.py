@@ -151,7 +151,7 @@ def test_complex_widths(width, w, dtype):
 
 def test_capture_of_a_call_whose_workspace_was_never_grown():
     """Paths that want more workspace than their fallback must not allocate under capture: a fresh
-    handle's complex solve, an order of the strip solver and a TRSV whose flags fit are captured."""
+    handle's complex solve and an order of the strip solver are captured."""
     for dtype, k, cols in ((np.complex128, 200, 20), (np.float64, 400, 2000)):
         A, B = oracle.nan_triangle_problem(k, "L", "L", "N", "N", k, cols, k, k, dtype)
         X = oracle.trsm("L", "L", "N", "N", 1.0, A, B)

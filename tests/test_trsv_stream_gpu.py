@@ -1,6 +1,7 @@
 """The streaming TRSV (trsv_stream.cuh) at the edges of its 128-row blocks, all combinations, both
 element types, increments and leading dimensions, against the oracle; the flag solve in a workspace
-that holds only its flags gives the same answer; a wait that runs out is reported."""
+that holds only its flags gives the same answer, also under capture; a wait that runs out is
+reported."""
 import ctypes
 import itertools
 
@@ -105,3 +106,61 @@ def test_rows_solved_before_a_bad_entry_of_a_stay_finite(pos, before, what, tran
     assert np.abs(out[:pos] - X).max() <= oracle.trsm_tolerance(np.float64, n) * max(1.0, np.abs(X).max())
     if what != "overflow":
         assert not np.isfinite(out[pos:]).any()
+
+
+@pytest.mark.parametrize("trans", "NT")
+@pytest.mark.parametrize("first_block", [1, 5])
+def test_wait_that_runs_out_is_reported(first_block, trans):
+    """The failure is made on the host: the claims start past the first blocks, whose x nothing then
+    publishes, and the waits are short.  The call returns, error 5 is reported once, and the handle
+    solves afterwards."""
+    n = 2048
+    A, B = oracle.nan_triangle_problem(2, "L", "L", trans, "N", n, 1, n, n, np.float64)
+    b = np.ascontiguousarray(B[:, 0])
+    L, code = rb.lib(), ctypes.c_int(-1)
+
+    def error(h):
+        assert L.rocblas_b200_get_device_error(h.value, ctypes.byref(code)) == 0
+        return code.value
+
+    keys = {b"wait_cycles_log2": 16, b"chain_first_item": first_block}
+    with rb.Handle() as h:
+        assert error(h) == 0
+        old = {}
+        try:
+            for key, value in keys.items():
+                assert L.rocblas_b200_get_tuning(key, ctypes.byref(code)) == 0
+                old[key] = code.value
+                assert L.rocblas_b200_set_tuning(key, value) == 0
+            _trsv(h, np.float64, "L", trans, "N", n, A, n, b, 1)
+        finally:
+            for key, value in old.items():
+                L.rocblas_b200_set_tuning(key, value)
+        assert error(h) == 5 and error(h) == 0
+        out = _trsv(h, np.float64, "L", trans, "N", n, A, n, b, 1)
+        X = oracle.trsm("L", "L", trans, "N", 1.0, A, B)[:, 0]
+        assert np.abs(out - X).max() <= oracle.trsm_tolerance(np.float64, n) * max(1.0, np.abs(X).max())
+        assert error(h) == 0
+
+
+def test_capture_with_a_workspace_of_flags():
+    """Under capture the workspace does not grow: a handle whose workspace is that of a short solve
+    captures a longer one as the flag solve."""
+    small, n = 256, 2048
+    A, B = oracle.nan_triangle_problem(4, "L", "L", "N", "N", n, 1, n, n, np.float64)
+    X = oracle.trsm("L", "L", "N", "N", 1.0, A, B)[:, 0]
+    s = torch.cuda.Stream()
+    with rb.Handle() as h, torch.cuda.stream(s):
+        h.set_stream(ctypes.c_void_p(s.cuda_stream))
+        _trsv(h, np.float64, "L", "N", "N", small, np.asfortranarray(A[:small, :small]), small,
+              np.ascontiguousarray(B[:small, 0]), 1)
+        dA, x = dm.to_device(A), torch.from_numpy(np.ascontiguousarray(B[:, 0])).cuda()
+        s.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            assert rb.lib().rocblas_dtrsv(h.value, rb.fill_lower, rb.operation_none, rb.diagonal_non_unit, n,
+                                          ctypes.c_void_p(dA.data_ptr()), n, ctypes.c_void_p(x.data_ptr()), 1) == 0
+        graph.replay()
+        s.synchronize()
+        out = x.cpu().numpy()
+    assert np.abs(out - X).max() <= oracle.trsm_tolerance(np.float64, n) * max(1.0, np.abs(X).max())
