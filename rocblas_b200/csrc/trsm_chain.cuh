@@ -927,7 +927,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) trsm_chain_kernel(ChainParam
 
         // ---- 3. X_b = inv(M_bb) T: chunks of the inverse through the ring, T resident ---------
         // k steps wholly outside the triangle of this warp's rows are skipped
-        double own[2][PT]; // (kOwn) this lane's rows' diagonal entries of the inverse
+        // (kOwn) this lane's rows' diagonal entries of the inverse; rows past its last chunk keep 0, as T
+        // is there
+        double own[2][PT] = {};
         auto   times_inverse = [&](auto ascending) {
             constexpr bool UP = decltype(ascending)::value; // descending: chunks, steps and a step's columns
             // the columns of a step that this lane holds (complex: an entry's two stay together)

@@ -181,21 +181,25 @@ def _substitution_80_bit(A, B, upper):
 @pytest.mark.parametrize("dtype", [np.float64, np.complex128])
 @pytest.mark.parametrize("w", [8, 16, 32, 64])
 @pytest.mark.parametrize("uplo", "LU")
-def test_rounding_error(width, uplo, w, dtype):
+@pytest.mark.parametrize("side,k,cols", [("L", 500, 150), ("R", 300, 1300)])
+def test_rounding_error(width, side, k, cols, uplo, w, dtype):
     """With a dominant diagonal a row's result is rounded three times: its right-hand side less the sum
     over the finished blocks, the reciprocal of its diagonal entry and their product plus the rest of
     the sum.  A rounding to nearest has a relative error of u / sqrt(3 m^2) in the mean square over
     mantissas m in [1, 2), 0.41 u; three give 0.71 u, and the bound leaves no room for a fourth
-    (0.82 u).  Complex: the reciprocal and the product have one more each, 0.91 u."""
+    (0.82 u).  Complex: the reciprocal and the product have one more each, 0.91 u.  (A block that is
+    substituted has one rounding per row before it; order 300 with 1300 rows from the right is checked
+    for blocks to substitute, and its last one is short.)"""
     assert width(w) == 0
-    k, cols = 500, 150
-    A, B = oracle.nan_triangle_problem(3, "L", uplo, "N", "N", k, cols, k, k, dtype)
+    m, n = (k, cols) if side == "L" else (cols, k)
+    A, B = oracle.nan_triangle_problem(3, side, uplo, "N", "N", m, n, k, m, dtype)
     with rb.Handle() as h:
         dA, dB = dm.to_device(A), dm.to_device(B)
-        dm.trsm(h, "L", uplo, "N", "N", k, cols, 1.0, dA, k, dB, k)
+        dm.trsm(h, side, uplo, "N", "N", m, n, 1.0, dA, k, dB, m)
         torch.cuda.synchronize()
-    X = _substitution_80_bit(A, B, uplo == "U")
-    d = dm.to_host(dB) - X
+    out = dm.to_host(dB)
+    X = _substitution_80_bit(A, B, uplo == "U") if side == "L" else _substitution_80_bit(A.T, B.T, uplo == "L").T
+    d = out - X
     error = np.sqrt((abs(d) ** 2).sum() / (abs(X) ** 2).sum())
     assert error <= (0.8 if dtype == np.float64 else 0.95) * 2.0**-53, error / 2.0**-53
 
