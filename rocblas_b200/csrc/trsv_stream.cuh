@@ -105,27 +105,21 @@ __global__ void __launch_bounds__(kTsThreads, 1) trsv_stream_kernel(const TrsvPa
         const int r0 = b * kTsNB, rows = min(kTsNB, p.n - r0);
 
         // ---- the diagonal block (identity past the matrix), inverted before any wait --------------
-        auto stage = [&]() {
-            for(int e = warp; e < kTsNB; e += kTsThreads / 32)
+        for(int e = warp; e < kTsNB; e += kTsThreads / 32)
 #pragma unroll
-                for(int u = 0; u < kTsNB / 32; ++u)
-                {
-                    const int  f = u * 32 + lane;
-                    const int  i = TR ? e : f, j = TR ? f : e; // lanes along A's contiguous direction
-                    double     v = 0.0;
-                    const bool one = i == j && (p.unit || i >= rows);
-                    if(j <= i && i < rows && !one)
-                        v = (double)M0[(r0 + i) * sI + (r0 + j) * sJ];
-                    X[j * kTrtriLd + i] = one ? 1.0 : v;
-                }
-            __syncthreads();
-        };
-        stage();
+            for(int u = 0; u < kTsNB / 32; ++u)
+            {
+                const int  f = u * 32 + lane;
+                const int  i = TR ? e : f, j = TR ? f : e; // lanes along A's contiguous direction
+                double     v = 0.0;
+                const bool one = i == j && (p.unit || i >= rows);
+                if(j <= i && i < rows && !one)
+                    v = (double)M0[(r0 + i) * sI + (r0 + j) * sJ];
+                X[j * kTrtriLd + i] = one ? 1.0 : v;
+            }
+        __syncthreads();
         if(!trtri_invert(X, Tm, false))
-        {
-            stage();
-            trtri_invert_rows(X, false);
-        }
+            trtri_invert_rows<T>(X, M0 + r0 * (sI + sJ), sI, sJ, rows, p.unit, false);
 
         // ---- the tiles left of it, in halves of 64 columns ----------------------------------------
         // no-trans: lane = 4 rows, warp = 8 columns; trans: lane = 2 columns, warp = 16 rows

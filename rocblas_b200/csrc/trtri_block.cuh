@@ -90,8 +90,7 @@ __device__ __forceinline__ void trtri_mma(double (&acc)[NT][4], const double* P,
 // the diagonal), in place, by 256 threads between two CTA barriers (the caller's before it, the
 // last of its own after it).  Tm: 64 columns of kTrtriLdT doubles.  Returns (in all threads) whether
 // everything it wrote is finite: if not, the zeros of a triangle may have met an infinity or NaN in a
-// product, and rows may not be finite that do not depend on it; the caller then stages the block again
-// for trtri_invert_rows.
+// product, and rows may not be finite that do not depend on it; trtri_invert_rows is for that case.
 __device__ __forceinline__ bool trtri_invert(double* X, double* Tm, bool zero_is_one)
 {
     bool finite = true;
@@ -170,19 +169,36 @@ __device__ __forceinline__ bool trtri_invert(double* X, double* Tm, bool zero_is
     return __syncthreads_and(finite) != 0;
 }
 
-// The same inverse with products over the triangles alone, so that what is not finite stays in the
-// rows from its own on, as in a substitution: column after column from the last one,
-// X21 = -X22 l21 / l11, thread = row.  About 0.1 ms.
-__device__ __noinline__ void trtri_invert_rows(double* X, bool zero_is_one)
+// The inverse at X again, of the triangle L0[i di + j dj] (j <= i < n; the identity past n), with
+// products over the triangles alone, so that what is not finite stays in the rows from its own on, as
+// in a substitution: column after column from the last one, X21 = -X22 l21 / l11, thread = row.  About
+// 0.1 ms; a function of its own, because the kernels around it are one pass through straight code and
+// this inside them cost 2 us.
+template <typename T>
+__device__ __noinline__ void trtri_invert_rows(double* X, const T* L0, int64_t di, int64_t dj, int n, bool unit,
+                                               bool zero_is_one)
 {
     const int r = threadIdx.x;
+    for(int e = r; e < kTrtriNB * kTrtriNB; e += kTrtriThreads)
+    {
+        const int i = e % kTrtriNB, j = e / kTrtriNB;
+        double    v = 0.0;
+        if(j < i && i < n)
+            v = (double)L0[i * di + j * dj];
+        else if(i == j)
+        {
+            v = i < n && !unit ? (double)L0[i * (di + dj)] : 1.0;
+            if(zero_is_one && v == 0.0)
+                v = 1.0;
+        }
+        X[j * kTrtriLd + i] = v;
+    }
+    __syncthreads();
     for(int c = kTrtriNB - 1; c >= 0; --c)
     {
-        const double* const l = X + c * kTrtriLd;
-        double              d = l[c], v = 0.0;
-        if(zero_is_one && d == 0.0)
-            d = 1.0;
-        const double rd = 1.0 / d;
+        const double* const l  = X + c * kTrtriLd;
+        const double        rd = 1.0 / l[c];
+        double              v  = 0.0;
         if(r > c && r < kTrtriNB)
         {
             for(int k = c + 1; k <= r; ++k)
@@ -227,52 +243,46 @@ __global__ void __launch_bounds__(kTrtriThreads) trtri_block_kernel(TrtriParams<
         take = i < bs && j < bs && (j < i || (i == j && !p.unit));
         return take ? A0 + sg * (i + (int64_t)j * lda) : A0;
     };
-    auto stage = [&]() {
-        if constexpr(std::is_same<T, double>::value)
-        {
+    if constexpr(std::is_same<T, double>::value)
+    {
 #pragma unroll
-            for(int c = 0; c < kTrtriNB / 8; ++c)
+        for(int c = 0; c < kTrtriNB / 8; ++c)
 #pragma unroll
-                for(int u = c / 4; u < kTrtriNB / 32; ++u)
-                {
-                    const int i = u * 32 + lane, j = c * 8 + warp;
-                    bool      take;
-                    const T*  src = source(i, j, take);
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(X + j * kTrtriLd + i)),
-                                 "l"(src), "r"(take ? 8 : 0)
-                                 : "memory");
-                }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-        }
-        else
-        {
-            // converted on the way: a row group's loads are all issued before its stores
-#pragma unroll
-            for(int u = 0; u < kTrtriNB / 32; ++u)
+            for(int u = c / 4; u < kTrtriNB / 32; ++u)
             {
-                T v[4 * (kTrtriNB / 32)];
-#pragma unroll
-                for(int c = 0; c < 4 * (u + 1); ++c)
-                {
-                    bool     take;
-                    const T* src = source(u * 32 + lane, c * 8 + warp, take);
-                    v[c]         = take ? *src : T(0);
-                }
-#pragma unroll
-                for(int c = 0; c < 4 * (u + 1); ++c)
-                    X[(c * 8 + warp) * kTrtriLd + u * 32 + lane] = (double)v[c];
+                const int i = u * 32 + lane, j = c * 8 + warp;
+                bool      take;
+                const T*  src = source(i, j, take);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(X + j * kTrtriLd + i)),
+                             "l"(src), "r"(take ? 8 : 0)
+                             : "memory");
             }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    else
+    {
+        // converted on the way: a row group's loads are all issued before its stores
+#pragma unroll
+        for(int u = 0; u < kTrtriNB / 32; ++u)
+        {
+            T v[4 * (kTrtriNB / 32)];
+#pragma unroll
+            for(int c = 0; c < 4 * (u + 1); ++c)
+            {
+                bool     take;
+                const T* src = source(u * 32 + lane, c * 8 + warp, take);
+                v[c]         = take ? *src : T(0);
+            }
+#pragma unroll
+            for(int c = 0; c < 4 * (u + 1); ++c)
+                X[(c * 8 + warp) * kTrtriLd + u * 32 + lane] = (double)v[c];
         }
-        __syncthreads();
-    };
-    stage();
+    }
+    __syncthreads();
 
     // unit diagonals and padding are staged as 0, which like a zero diagonal entry is read as 1
     if(!trtri_invert(X, Tm, true))
-    {
-        stage();
-        trtri_invert_rows(X, true);
-    }
+        trtri_invert_rows<T>(X, A0, sg, sg * lda, bs, p.unit, true);
 
     // ---- write inv(A_block) (bs x bs, ld = ldinv), zeros in the opposite triangle ----
     T* const out0 = p.upper ? out + (int64_t)(bs - 1) * (p.ldinv + 1) : out;
