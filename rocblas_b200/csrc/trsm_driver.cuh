@@ -390,6 +390,36 @@ enum class Algo
     recursive
 };
 
+// One system of an order that the one-CTA solvers take, with many strips of 32 columns: is the chain
+// faster?  It has eight MMA warps per SM and levels, but pads the order to 128-row blocks and pays for
+// the inverses and a hand-off per block; the strip solver runs four strips per SM at once in little
+// more time than one, the complex one-CTA solver one strip (FP64) or two.  Measured on one B200, chain
+// against one-CTA solver, us with the copy of the right-hand sides, side left:
+//   FP32   order 257: 1200 columns 52 / 59, 2000 61 / 60, 4000 89 / 62, 8192 105 / 66, 20000 178 / 140
+//          order 290: 2000 62 / 67, 4000 74 / 68, 8192 109 / 75, 20000 185 / 158
+//          order 330: 4000 76 / 84, 6000 95 / 94, 8192 113 / 93, 12000 130 / 111, 20000 192 / 198
+//          order 384: 6000 93 / 99, 12000 129 / 121, 20000 193 / 208; 512: 8192 139 / 160, 20000 293 / 349
+//   FP64   the same within 10% (order 256 with 4096 columns: 52 / 43)
+//   complex FP64  order 129: 2000 90 / 103, 4000 120 / 103, 8000 (two waves of strips) 149 / 197
+//          order 150: 2000 95 / 105, 4000 111 / 106; 180: 4000 134 / 140; 256: 2000 88 / 209
+//          order 128: 2000 75 / 67
+//   complex FP32  order 129: 1184 69 / 69, 2000 82 / 70, 4000 113 / 70, 16000 228 / 178
+//          order 180: 1184 87 / 92, 2000 103 / 93, 8000 168 / 128, 16000 230 / 238
+//          order 210: 3000 111 / 115, 4000 129 / 115, 8000 204 / 158; 256: 4000 119 / 136
+template <typename T>
+static bool chain_beats_one_cta(int k, int64_t strips, int sms)
+{
+    if constexpr(is_cplx<T>::value)
+    {
+        if(k <= 128)
+            return false;
+        if(sizeof(T) > 8)
+            return k > 160 || strips * 2 <= sms || strips > sms;
+        return k > 224 || strips * (k > 192 ? 3 : 8) <= (int64_t)sms * 2;
+    }
+    return k > 352 || (k > 256 && strips * (k > 320 ? 3 : 8) <= (int64_t)sms * 4);
+}
+
 template <typename T>
 static Algo choose_algo(const TrsmProblem<T>& pr)
 {
@@ -399,15 +429,10 @@ static Algo choose_algo(const TrsmProblem<T>& pr)
         return Algo::recursive;
     if(k <= t.block_always_k)
         return Algo::block;
-    // One system with many strips: above 256 rows the chain's four MMA warps more per SM and its
-    // levels beat the strip solver's one CTA per strip (512 x 2048: 67 against 112 us, 512 x 8192
-    // 140 against 151, 300 x 4096 the same), below it they do not (256 x 4096: 52 against 43).
-    // Complex strips are solved by a slower one-CTA solver (256 x 2000: 201 against 87 us on the
-    // chain, 129 against 81 in single precision; at 128 x 2000 75 against 67 and 53 against 58).
-    if(pr.chain_small && pr.batch == 1 && k > (is_cplx<T>::value ? 128 : 256))
-        return Algo::recursive;
     const int64_t ncols   = pr.side_left ? pr.n : pr.m;
     const int64_t nstrips = ceil_div(ncols, kBsW) * (int64_t)pr.batch;
+    if(pr.chain_small && pr.batch == 1 && chain_beats_one_cta<T>(k, nstrips, pr.sm_count))
+        return Algo::recursive;
     return nstrips * 100 >= (int64_t)pr.sm_count * t.block_min_strips_pct ? Algo::block
                                                                          : Algo::recursive;
 }

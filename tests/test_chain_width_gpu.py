@@ -227,3 +227,29 @@ def test_inverse_block_of_a_non_finite_entry(i, j, bad, dtype):
             assert not np.isfinite(X[i, j]) and (np.triu(X, 1) == 0).all()
             Y = np.linalg.inv(T[:i, :i].astype(dtype).astype(np.float64))
             assert np.abs(X[:i, :i] - Y).max() <= 4 * n * np.finfo(dtype).eps
+
+
+@pytest.mark.parametrize("dtype,lines", [
+    (np.float64, [(257, 2), (320, 2), (321, 0.75), (352, 0.75), (353, 0.75)]),
+    (np.float32, [(320, 2), (352, 0.75)]),
+    (np.complex128, [(129, 2), (160, 1), (161, 2)]),
+    (np.complex64, [(129, 4), (192, 4), (193, 1.5), (224, 1.5), (225, 1.5)])])
+def test_both_sides_of_the_line_between_chain_and_one_cta_solvers(dtype, lines):
+    """(order, d): the line is at SMs / d strips of 32 columns."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    u = np.finfo(dtype).eps / 2
+    with rb.Handle() as h:
+        for k, d in lines:
+            for cols in (int(sms / d) * 32, int(sms / d) * 32 + 1):
+                for side in "LR":
+                    m, n = (k, cols) if side == "L" else (cols, k)
+                    A, B = oracle.nan_triangle_problem(k, side, "L", "N", "N", m, n, k, m, dtype)
+                    dA, dB = dm.to_device(A), dm.to_device(B)
+                    dm.trsm(h, side, "L", "N", "N", m, n, 1.0, dA, k, dB, m)
+                    M = torch.tril(dA.mT)
+                    # residual of a backward stable solve: 2 k u of |M| |X| (complex: twice as many products)
+                    if side == "L":
+                        R, bound = (M @ dB.mT - dm.to_device(B).mT).abs(), M.abs() @ dB.mT.abs()
+                    else:
+                        R, bound = (dB.mT @ M - dm.to_device(B).mT).abs(), dB.mT.abs() @ M.abs()
+                    assert (R <= (4 if np.iscomplexobj(A) else 2) * k * u * bound).all(), (k, cols, side)
