@@ -1234,7 +1234,8 @@ __global__ void vb_copy_invalid_kernel(const int* invalid, rocblas_int* out)
 
 static_assert(sizeof(VbProblem) == sizeof(rocblas_b200_trsm_problem), "descriptor layout");
 
-// Persistent strip-solver launch over one queue of systems up to kmax.
+// Persistent launch over one queue of systems up to kmax: the strip solver, whose launch is the same
+// for every kmax, or one strip per warp where kmax is at most kVbWarpMaxK.
 template <typename T>
 void launch_vb_queue(rocblas_handle h, const VbParams<T>& p, int kmax)
 {

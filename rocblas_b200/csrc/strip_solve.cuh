@@ -34,8 +34,8 @@
 //
 // Measured (one B200, against the solver with the strip in shared memory and one-warp
 // substitutions; passes with the copy of the right-hand sides): 4096 systems of 128 x 32 in FP64
-// 515 -> 211 us, 20,000 uneven systems 4.39 -> 2.01 ms, one 96 x 24 system 18.6 -> 14.3 us.  What
-// bounds the uniform batch is the L1 data pipe (74% busy; DRAM 37%, DMMA 37%): every warp reads the
+// 515 -> 209 us, 20,000 uneven systems 4.39 -> 2.00 ms, one 96 x 24 system 18.5 -> 12.3-14.3 us.  What
+// bounds the uniform batch is the L1 data pipe (75% busy; DRAM 40%, DMMA 40%): every warp reads the
 // whole triangle for its 8 right-hand sides.
 #pragma once
 #include <type_traits>
@@ -70,9 +70,9 @@ constexpr int kSsW       = 32;  // right-hand sides per CTA
 constexpr int kSsThreads = 128; // 8 right-hand sides per warp
 constexpr int kSsPanel   = 32;  // columns of M per panel
 constexpr int kSsMaxK    = 512;
-// Super-blocks of 64 rows, two panels in the ring, registers for four CTAs per SM: 211 us for 4096
-// systems of 128 x 32 and 2010 us for 20,000 uneven ones (five CTAs 224 and 2139; 128 rows, which
-// leave three, 242 and 2350; three and four panels were no faster).
+// Super-blocks of 64 rows, two panels in the ring, registers for four CTAs per SM, measured side by
+// side: 211 us for 4096 systems of 128 x 32 and 2010 us for 20,000 uneven ones (five CTAs 224 and
+// 2139; 128 rows, which leave three, 242 and 2350; three and four panels were no faster).
 constexpr int kSsRT   = 8;
 constexpr int kSsNS   = 2;
 constexpr int kSsCtas = 4;

@@ -31,9 +31,10 @@
 // copies start while the MMA warps finish the current one.
 //
 // Measured (one B200, FP64, against the same chain with copies by the MMA warps and 64-column
-// strips): 3001 x 77 with invA 716 -> 156 us, 8192 x 512 2.31 -> 1.41 ms (24.4 TFLOP/s), 8192 x
-// 8192 23.1 -> 17.7 ms (31.1 TFLOP/s, 0.84 of the tensor pipe's 37.2).  Few right-hand sides are
-// bound by the chain: 5.7 us per block at 8 columns, of which the two products take 1.6 us.
+// strips): 3001 x 77 with invA 716 -> 158 us, 8192 x 512 2.31 -> 1.40 ms (24.5 TFLOP/s), 8192 x
+// 8192 23.1 -> 17.6 ms (31.2 TFLOP/s, 0.84 of the tensor pipe's nominal 37.2 and 0.88 of the 35.5
+// that cuBLAS DGEMM reaches).  Few right-hand sides are bound by the chain: 5.8 us per block at 8
+// columns, of which the two products take 1.6 us.
 //
 // Every wait is bounded (ChainParams::wait_cycles, about a second); on timeout the kernel
 // records error code 4, all roles run out without waiting, and the CTA stops, so a wrong flag

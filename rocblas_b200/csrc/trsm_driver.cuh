@@ -6,8 +6,10 @@
 // among five algorithms and, for large k, runs a host loop of two GEMMs per 128-row block;
 // for m=16384, n=4096 that is 256 GEMMs whose outputs are only 128 rows tall.  Here:
 //
-//   * k <= 512 and enough strips (or k <= 128): the one-CTA block solver (block_solve.cuh).
-//   * otherwise: a recursive blocked solve on the 128-block grid of A.  A node of
+//   * k <= 128, or k <= 512 and enough strips: a one-CTA solver per strip of 32 right-hand sides
+//     (strip_solve.cuh; complex: block_solve.cuh), unless the chain is faster (chain_beats_one_cta).
+//   * otherwise the chain of 128-row blocks in one launch (trsm_chain.cuh, use_chain), or where
+//     it does not apply: a recursive blocked solve on the 128-block grid of A.  A node of
 //     blocks [b0, b1) splits at the middle block bm and runs
 //         solve(first half, alpha); B2 := alpha_or_1 * B2 - op(A)21 * X1; solve(second half, 1)
 //     so that half of all flops land in one large GEMM at the top level and the chain of

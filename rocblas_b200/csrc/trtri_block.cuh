@@ -15,8 +15,8 @@
 //
 // The kernel is a chain of short steps (a solve waits for it before its first block), so it is
 // bound by latency: copies that are all in flight at once, seven CTA barriers, and no index
-// arithmetic beyond constants: 14 us for up to 148 FP64 blocks of 128 where the version on 32 x 32
-// tiles with computed tile indexes took 42 us (a third of a 512 x 256 solve).
+// arithmetic beyond constants: 14 us for up to 148 FP64 blocks of 128 (FP32 16) where the version on
+// 32 x 32 tiles with computed tile indexes took 42 us (a third of a 512 x 256 solve).
 //
 // Diagonal semantics follow rocblas_custom_trtri_device (rocblas_trtri.hpp:128-141):
 // diag == unit reads no diagonal and uses 1; a zero non-unit diagonal entry is treated as 1.

@@ -9,12 +9,12 @@
 //      its triangle order k (k <= 32, 64, 128, 256, 512), counts its work items (strips of 32
 //      right-hand sides) and writes, per class, the exclusive prefix sum of those counts
 //      (problems of other classes count 0);
-//   2. per class, a persistent kernel (grid = SMs x resident CTAs, shared memory sized for
-//      that class's largest k, so small systems run many CTAs per SM) pulls work-item indices
+//   2. per class, a persistent kernel (grid = SMs x resident CTAs) pulls work-item indices
 //      from the class's device-side queue head (one atomicAdd per item), maps an item to its
 //      (problem, strip) by binary search over the class's prefix sum, and runs the one-CTA
-//      strip solver (block_solve.cuh) on it; the k <= 32 class runs one strip per warp
-//      instead (vb_warp_kernel).  There is no inter-CTA waiting, so no wait can hang.
+//      strip solver (strip_solve.cuh, whose shared memory does not depend on k) on it; the
+//      k <= 32 class runs one strip per warp instead (vb_warp_kernel).  There is no inter-CTA
+//      waiting, so no wait can hang.
 // All launches are stream-ordered and capturable in a CUDA graph.
 #pragma once
 #include "strip_solve.cuh"
